@@ -36,8 +36,29 @@ QFD_HD uint32_t red64(uint64_t v) {  // v < 2^48
   uint32_t g = uint32_t((f & 0xffffu) + 15ull * (f >> 16));
   return red32(g);
 }
+QFD_HD uint32_t umin32(uint32_t a, uint32_t b) { return a < b ? a : b; }
 QFD_HD uint32_t addp(uint32_t a, uint32_t b) { uint32_t s = a + b; return s >= P ? s - P : s; }
 QFD_HD uint32_t subp(uint32_t a, uint32_t b) { return a >= b ? a - b : a + P - b; }
+// Four unsigned byte products added to c, and a byte permute (host forms for
+// the CPU check of this header).
+QFD_HD uint32_t dp4u(uint32_t a, uint32_t b, uint32_t c) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 610
+  return __dp4a(a, b, c);
+#else
+  for (int i = 0; i < 32; i += 8) c += ((a >> i) & 0xffu) * ((b >> i) & 0xffu);
+  return c;
+#endif
+}
+QFD_HD uint32_t bytes(uint32_t a, uint32_t b, uint32_t sel) {
+#if defined(__CUDA_ARCH__)
+  return __byte_perm(a, b, sel);
+#else
+  const uint64_t v = uint64_t(b) << 32 | a;
+  uint32_t r = 0;
+  for (int i = 0; i < 4; ++i) r |= uint32_t(v >> (8 * (sel >> (4 * i) & 7)) & 0xffu) << (8 * i);
+  return r;
+#endif
+}
 
 QFD_HD Fr load(const Fe* p) {
   uint4 u = *reinterpret_cast<const uint4*>(p);
@@ -76,48 +97,82 @@ QFD_HD uint32_t red_signed(int64_t v) {
   u = (u & 0xffffu) + 15u * (u >> 16);
   return red40(u);
 }
-QFD_HD Fr mul(const Fr& a, const Fr& b) {
-  // A loop's fixed factor goes second, so that 17 * b is computed once.
-  // X^8 = 17: the wrap-around products take 17 * b_j (< 2^21, unreduced), so
-  // output coefficient k is one sum of eight products a_i * b'_j < 2^37,
-  // accumulated with 64-bit multiply-adds (< 2^40) and reduced once.
-  uint32_t b17[8];
+// The product's output coefficients, raw: coefficient k is the sum over i of
+// a_i w_(k - i), w_j = b_j and, for the wrap-around X^8 = 17, w_(j - 8) = 17 b_j
+// mod p.  All operands are 16 bits, so their byte planes multiply by dp4a,
+// four products each: with s0, s1, s2 the sums of the low-low, mixed and
+// high-high byte products, the coefficient is s0 + 2^8 s1 + 2^16 s2, and 2^16
+// = 15 keeps it in 32 bits (below 2^28.1).  64 dp4a take 1.40 clocks per
+// product and SM with the reductions (measured on B200, operands in
+// registers); 64 widening multiply-adds, which issue at half that rate each,
+// took 2.04.
+struct Raw {
+  uint32_t c[8];
+};
+QFD_HD Raw mul_raw(const Fr& a, const Fr& b) {
+  // Bytes a_0..a_3 and a_4..a_7, low and high.
+  uint32_t al[2], ah[2];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) b17[j] = 17u * b.c[j];
-  uint64_t r[8];
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t x = bytes(a.c[4 * i], a.c[4 * i + 1], 0x5410), y = bytes(a.c[4 * i + 2], a.c[4 * i + 3], 0x5410);
+    al[i] = bytes(x, y, 0x6420);
+    ah[i] = bytes(x, y, 0x7531);
+  }
+  // w_7, w_6, .., w_0, w_-1, .., w_-8 as bytes.  A loop's fixed factor goes
+  // second, so that these are formed once.
+  uint32_t wl[4], wh[4];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) r[k] = 0;
+  for (int i = 0; i < 4; ++i) {
+    uint32_t v[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (i + j < 8) r[i + j] += uint64_t(a.c[i]) * b.c[j];
-      else r[i + j - 8] += uint64_t(a.c[i]) * b17[j];
+    for (int j = 0; j < 4; ++j) {
+      v[j] = b.c[7 - ((4 * i + j) & 7)];
+      if (i >= 2) {
+        v[j] *= 17u;
+        v[j] -= (v[j] >> 16) * P;
+        v[j] = umin32(v[j], v[j] - P);
+      }
     }
+    const uint32_t x = bytes(v[0], v[1], 0x5410), y = bytes(v[2], v[3], 0x5410);
+    wl[i] = bytes(x, y, 0x6420);
+    wh[i] = bytes(x, y, 0x7531);
+  }
+  Raw r;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    // The window w_k, w_(k - 1), .., w_(k - 7).
+    const int q = (7 - k) >> 2, sh = (7 - k) & 3;
+    const uint32_t sel = sh == 1 ? 0x4321u : (sh == 2 ? 0x5432u : 0x6543u);
+    const uint32_t l0 = sh ? bytes(wl[q], wl[q + 1], sel) : wl[q], l1 = sh ? bytes(wl[q + 1], wl[q + 2], sel) : wl[q + 1];
+    const uint32_t h0 = sh ? bytes(wh[q], wh[q + 1], sel) : wh[q], h1 = sh ? bytes(wh[q + 1], wh[q + 2], sel) : wh[q + 1];
+    const uint32_t s0 = dp4u(al[1], l1, dp4u(al[0], l0, 0u)), s2 = dp4u(ah[1], h1, dp4u(ah[0], h0, 0u));
+    const uint32_t s1 = dp4u(al[1], h1, dp4u(al[0], h0, dp4u(ah[1], l1, dp4u(ah[0], l0, 0u))));
+    r.c[k] = s2 * 15u + s0 + s1 * 256u;
+  }
+  return r;
+}
+QFD_HD Fr mul(const Fr& a, const Fr& b) {
+  const Raw r = mul_raw(a, b);
   Fr out;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) out.c[k] = red40(r[k]);
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t f = r.c[k] - (r.c[k] >> 16) * P;  // below 2^16 + 15 * 2^12.1 < 2p
+    out.c[k] = umin32(f, f - P);
+  }
   return out;
 }
-// Lazy sums of products: a product adds at most eight terms below 2^36.1 to
-// each raw coefficient (below 2^39.1), so a 64-bit accumulator takes 2^24
-// products before it could overflow; it is reduced once at the end (two
-// folds of 2^16 = 15 bring any u64 below 2^40, then red40).
+// Lazy sums of products: a raw product is below 2^28.1 per coefficient, so a
+// 64-bit accumulator takes 2^24 products with room to spare; it is reduced
+// once at the end (two folds of 2^16 = 15 bring any u64 below 2^40, then
+// red40).
 struct Acc {
   uint64_t c[8];
 };
 QFD_HD Acc acc_zero() { Acc r; for (int k = 0; k < 8; ++k) r.c[k] = 0; return r; }
 QFD_HD void mul_acc(Acc& r, const Fr& a, const Fr& b) {
-  uint32_t b17[8];
+  const Raw t = mul_raw(a, b);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) b17[j] = 17u * b.c[j];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (i + j < 8) r.c[i + j] += uint64_t(a.c[i]) * b.c[j];
-      else r.c[i + j - 8] += uint64_t(a.c[i]) * b17[j];
-    }
+  for (int k = 0; k < 8; ++k) r.c[k] += t.c[k];
 }
 QFD_HD Fr acc_reduce(const Acc& r) {
   Fr out;
@@ -142,8 +197,15 @@ QFD_HD Fr unpack_fe(uint4 u) {
   v.c[4] = u.z & 0xffffu; v.c[5] = u.z >> 16; v.c[6] = u.w & 0xffffu; v.c[7] = u.w >> 16;
   return v;
 }
+QFD_HD uint32_t pack16(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return __byte_perm(a, b, 0x5410);
+#else
+  return a | (b << 16);
+#endif
+}
 QFD_HD uint4 pack_fe(const Fr& r) {
-  return make_uint4(r.c[0] | (r.c[1] << 16), r.c[2] | (r.c[3] << 16), r.c[4] | (r.c[5] << 16), r.c[6] | (r.c[7] << 16));
+  return make_uint4(pack16(r.c[0], r.c[1]), pack16(r.c[2], r.c[3]), pack16(r.c[4], r.c[5]), pack16(r.c[6], r.c[7]));
 }
 
 // Planar transform tiles use lazy reduction: a value entering level l of a
