@@ -224,6 +224,24 @@ QFD_HD uint32_t tile_final(uint32_t v) {
   return f >= P ? f - P : f;
 }
 
+// Limb sums of the tensor-core transforms: s[2i] and s[2i + 1] hold (as s32)
+// sums of at most 128 signed terms of coefficient i's low and high byte.  The
+// coefficient t = s[2i] + 256 s[2i + 1] is within 128 (p - 1) of zero; adding
+// 128 p makes it an unsigned value below 2^24, one fold of 2^16 = 15 (as a
+// multiply-add, t - 65521 (t >> 16)) brings it below 2 p.
+#if defined(__CUDACC__)
+__device__ __forceinline__ Fr limb_sums(const uint32_t (&s)[16], uint32_t c256) {
+  Fr r;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t t = s[2 * i + 1] * c256 + (s[2 * i] + 128u * P);
+    const uint32_t f = t - (t >> 16) * P;
+    r.c[i] = __viaddmin_u32(f, 0u - P, f);
+  }
+  return r;
+}
+#endif
+
 // small signed integer -> canonical F_65521 (field.rs:24-26)
 QFD_HD uint32_t small(int v) { return v < 0 ? uint32_t(v + int(P)) : uint32_t(v); }
 // Eight signed 8-bit weights (8 bytes) to the packed element.
@@ -233,5 +251,22 @@ QFD_HD Fr weights_to_fr(uint2 raw) {
   for (int k = 0; k < 8; ++k) r.c[k] = small(int(int8_t(((k < 4 ? raw.x : raw.y) >> (8 * (k & 3))) & 0xffu)));
   return r;
 }
+
+// The same packed: bytes sign-extended in 16-bit pairs, less 15 where negative
+// (v + p = v - 15 mod 2^16, and no borrow leaves the half).
+#if defined(__CUDACC__)
+__device__ __forceinline__ uint4 pack_weights(uint2 raw) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t b = i < 2 ? raw.x : raw.y;
+    uint32_t v, sign;  // a selector nibble of 8 + j replicates byte j's sign
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(v) : "r"(b), "r"(i & 1 ? 0xb3a2u : 0x9180u));
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(sign) : "r"(b), "r"(i & 1 ? 0xbbaau : 0x9988u));
+    w[i] = v - (sign & 0x000f000fu);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+#endif
 
 }  // namespace qfd

@@ -7,6 +7,7 @@
 #include "kernels/dot_mma.cuh"
 #if !defined(QF_FIELD_KB)
 #include "kernels/imma_f65521.cuh"
+#include "kernels/transform_mma.cuh"
 #endif
 #include "intops.h"
 
@@ -158,6 +159,10 @@ std::vector<F> DeviceCodeword::entries() const {
   return h;
 }
 
+// The tensor-core transform passes (F65521), below.
+static void configure_transforms();
+static void check_transforms();
+
 // Planar tile kernels take up to 2^kMaxTileLog elements (128 KiB of shared
 // memory); the opt-in is set once per device.
 static void configure_tile_kernels() {
@@ -180,6 +185,7 @@ static void configure_tile_kernels() {
   // 38 KiB of static shared memory plus the 32 KiB weight double buffer.
   set_smem(qfd::k_eq_project_blocks, qfd::kEqWeightSmem);
 #endif
+  configure_transforms();
   done.insert(dev);
 }
 
@@ -508,6 +514,123 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
   }
 }
 
+#if !defined(QF_FIELD_KB)
+// ---------------------------------------------------------------- tensor-core transform passes
+// Codewords of at least 2^23 message entries run their tile passes and the
+// strided passes of six levels or more on the tensor cores
+// (kernels/transform_mma.cuh).  Measured on B200, F65521, against the
+// butterfly kernels, ms per pass:
+//   2^25 entries  WHT of 9 strided levels 0.248 / 0.320, Mobius + WHT 0.500 /
+//                 0.563, WHT alpha WHT 0.731 (13 levels each) / 0.815 (12),
+//                 Mobius tile of an element vector 0.223 (13) / 0.309 (12),
+//                 of weights 0.285 (13) / 0.342 (12)
+//   2^23          0.078 / 0.083, -, 0.203 / 0.213, 0.072 / 0.088, 0.090 / 0.095
+//   2^22          0.053 / 0.045, -, 0.127 / 0.113: 3.5 tiles per SM leave the
+//                 chain of a tile's stages exposed
+//   2^25, 5 levels  0.25 / 0.22: one stage, bound by HBM either way
+// A KoalaBear pass costs the same time here, but its butterflies work on half
+// as many coefficients (0.26, 0.45, 0.59 at 2^25): it keeps them.
+static constexpr int kMmaMinLogm = 23;
+static bool mma_transforms(int logm, int logR) { return logm >= kMmaMinLogm && logR >= qfd::kTcTileLog; }
+
+// A wait that gave up in k_transform: one flag per process in host memory
+// that the device can write.
+static int* transform_error() {
+  static int* flag = [] {
+    int* p = nullptr;
+    QF_CK(cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    *p = 0;
+    return p;
+  }();
+  return flag;
+}
+static void check_transforms() {
+  if (*static_cast<volatile int*>(transform_error())) fail(QF_E_CUDA, "CUDA: a transform pass gave up waiting");
+}
+
+template <int CFG, int SRC, int OP1, int OP2, int MID, bool HASY>
+struct Transform {
+  static constexpr int kMats = (HASY ? 2 : 1) * (OP2 >= 0 && OP1 != OP2 ? 2 : 1);
+  static void configure() { set_smem(qfd::k_transform<CFG, SRC, OP1, OP2, MID, HASY>, qfd::tc_smem(kMats)); }
+  static void run(cudaStream_t s, qfd::TcPass& p) {
+    p.error = transform_error();
+    qfd::k_transform<CFG, SRC, OP1, OP2, MID, HASY><<<tile_grid(p.n_tiles), qfd::tc_threads(SRC), qfd::tc_smem(kMats), s>>>(p);
+  }
+};
+using PackMobius = Transform<qfd::kTileCfg, qfd::kTcWeights, qfd::kMobius, -1, qfd::kMidNone, true>;
+using CopyMobius = Transform<qfd::kTileCfg, qfd::kTcLinear, qfd::kMobius, -1, qfd::kMidNone, true>;
+using WhtAlphaWht = Transform<qfd::kTileCfg, qfd::kTcElements, qfd::kWht, qfd::kWht, qfd::kMidAlpha, true>;
+using StridedWht = Transform<qfd::kStridedCfg, qfd::kTcElements, qfd::kWht, -1, qfd::kMidNone, true>;
+using MobiusWht = Transform<qfd::kStridedCfg, qfd::kTcElements, qfd::kMobius, qfd::kWht, qfd::kMidStore, true>;
+using MobiusWhtShort = Transform<qfd::kStridedCfg, qfd::kTcElements, qfd::kMobius, qfd::kWht, qfd::kMidStore, false>;
+
+static void configure_transforms() {
+  transform_error();
+  PackMobius::configure();
+  CopyMobius::configure();
+  WhtAlphaWht::configure();
+  StridedWht::configure();
+  MobiusWht::configure();
+  MobiusWhtShort::configure();
+}
+
+// Codeword stride of logical index bit `bit` (message half).
+static uint32_t index_stride(int bit, int logR) { return bit < logR ? 1u << bit : 1u << (bit + 1); }
+// The low 13 index bits of a tile, all with a level.
+static qfd::TcPass tile_pass(const void* src, Fe* dst, int logR, int logm) {
+  qfd::TcPass p{};
+  p.src = src;
+  p.dst = dst;
+  p.logR = logR;
+  p.k = qfd::kTcTileLog;
+  p.c256 = 256;
+  p.n_tiles = uint32_t(1) << (logm - qfd::kTcTileLog);
+  for (int j = 0; j < qfd::kTcTileLog; ++j) p.stride[j] = index_stride(j, logR);
+  p.mask_x = 0x7f;
+  p.mask_y = 0x7e;  // slot 0 is taken by stage X
+  return p;
+}
+// Levels [lo, lo + k) and the low 13 - k index bits as runs.  The shared slots
+// 0 and 1 are the shortest runs; with four run bits or more slot 2 comes next,
+// so that stage X's lanes cover 128 bytes; slot 12 (in neither stage's
+// contraction) is a run too.  A single stage (k <= 5) is X, its levels in its
+// upper slots.
+static qfd::TcPass strided_pass(const void* src, Fe* dst, int logR, int logm, int lo, int k) {
+  static constexpr int kRuns[13] = {0, 1, 2, 12, 3, 7, 8, 4, 9, 5, 10, 6, 11}, kRuns3[3] = {0, 1, 12};
+  static constexpr int kContractY[7] = {0, 1, 7, 8, 9, 10, 11};
+  const int runs = qfd::kTcTileLog - k;
+  check(k >= 1 && k <= 10 && lo >= runs, "strided transform pass");
+  qfd::TcPass p{};
+  p.src = src;
+  p.dst = dst;
+  p.logR = logR;
+  p.lo = lo;
+  p.k = k;
+  p.cb = runs;
+  p.c256 = 256;
+  p.n_tiles = uint32_t(1) << (logm - qfd::kTcTileLog);
+  bool used[13] = {};
+  auto place = [&](int slot, int bit) {
+    used[slot] = true;
+    p.stride[slot] = index_stride(bit, logR);
+  };
+  for (int j = 0; j < runs; ++j)
+    place(k <= 5 ? (j < 7 - k ? j : j + k) : (runs == 3 ? kRuns3[j] : kRuns[j]), j);
+  for (int j = 0, slot = 0; j < k; ++j) {
+    while (used[slot]) ++slot;
+    place(slot, lo + j);
+    if (slot < 7) p.mask_x |= 1u << slot;
+    else
+      for (int q = 0; q < 7; ++q)
+        if (kContractY[q] == slot) p.mask_y |= 1u << q;
+  }
+  return p;
+}
+#else
+static void configure_transforms() {}
+static void check_transforms() {}
+#endif
+
 // The transform passes of one codeword (2^logm message entries in 2^(logm -
 // logR) columns of R = 2^logR rows, message half at cw, parity at cw + R).
 // On entry the message half holds the packed message with its Mobius levels
@@ -552,6 +675,51 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
     }
     return;
   }
+#if !defined(QF_FIELD_KB)
+  if (mma_transforms(logm, logR)) {
+    // The same passes over tiles of 13 bits on the tensor cores; spans of five
+    // levels or fewer are bound by HBM and stay with the butterflies.
+    constexpr int kT = qfd::kTcTileLog;
+    check(!mobius || mob_from == kT, "the Mobius tile pass covers bits 0..12");
+    const uint64_t n = uint64_t(1) << logm;
+    const int top = std::min(logR, kT + 10), k = top - kT;
+    auto wht = [&](const Fe* src, int from) {  // levels [from, logR) into the parity
+      while (from < logR) {
+        const int span = logR - from, levels = span > 10 ? span / 2 : span;
+        if (levels <= 5) {
+          strided_passes<qfd::kWht>(s, src, par, logR, logm, from, from + levels, timed, allow_tuning);
+        } else {
+          qfd::TcPass p = strided_pass(src, par, logR, logm, from, levels);
+          launch(s, timed, "k_transform_wht", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0),
+                 [&] { StridedWht::run(s, p); });
+        }
+        src = par;
+        from += levels;
+      }
+    };
+    if (mobius) {
+      strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, top, logm, timed, allow_tuning);
+      if (k > 0) {
+        qfd::TcPass p = strided_pass(msg, par, logR, logm, kT, k);
+        p.mid = msg;
+        launch(s, timed, "k_transform_mobius_wht", 3 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, k > 5 ? 4 : 2, 0), [&] {
+          if (k > 5) MobiusWht::run(s, p);
+          else MobiusWhtShort::run(s, p);
+        });
+      }
+      wht(par, top);
+    } else {
+      wht(msg, kT);
+    }
+    qfd::TcPass p = tile_pass(k > 0 ? par : msg, par, logR, logm);
+    p.alpha = alpha;
+    p.col_log = logm - logR;
+    launch(s, timed, "k_transform_wht_alpha_wht", 2 * n * 16 + uint64_t(R) * 16, qf_intops::transform_ops(kOps, n, 0, 0, 4, 1),
+           [&] { WhtAlphaWht::run(s, p); });
+    wht(par, kT);
+    return;
+  }
+#endif
   constexpr int kT = qfd::kMaxTileLog;
   check(!mobius || mob_from == kT, "the Mobius tile pass covers bits 0..11");
   const int top = std::min(logR, kT + 10);  // fused span [kT, top)
@@ -589,6 +757,52 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
                src, par, alpha, logR, tiles);
          });
   strided_passes<qfd::kWht>(s, par, par, logR, logm, kT, logR, timed, allow_tuning);
+}
+
+// Levels a codeword's first pass takes off the Mobius transform: one tile's.
+static int first_mobius_levels(int logm, int logR) {
+#if !defined(QF_FIELD_KB)
+  if (mma_transforms(logm, logR)) return qfd::kTcTileLog;
+#endif
+  (void)logR;
+  return std::min(qfd::kMaxTileLog, logm);
+}
+// Packed weights of one block (from entry src_base of the `active` at bva)
+// with their first Mobius levels into the message half at cw.
+static void pack_mobius(cudaStream_t s, bool timed, const W* bva, uint64_t active, uint64_t src_base, Fe* cw, int logR, int logm) {
+  check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
+  const int l0 = first_mobius_levels(logm, logR);
+  const uint64_t n = uint64_t(1) << logm, bytes = n * (F::kLanes * sizeof(W) + 16);
+#if !defined(QF_FIELD_KB)
+  if (mma_transforms(logm, logR)) {
+    qfd::TcPass p = tile_pass(bva, cw, logR, logm);
+    p.active = active;
+    p.src_base = src_base;
+    launch(s, timed, "k_transform_pack_mobius", bytes, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0), [&] { PackMobius::run(s, p); });
+    return;
+  }
+#endif
+  const uint32_t tiles = uint32_t(n >> l0);
+  launch(s, timed, "k_pack_mobius_tile", bytes, qf_intops::transform_ops(kOps, n, 0, l0, 1, 0), [&] {
+    qfd::k_pack_mobius_tile<<<tile_grid(tiles), qfd::kTileThreads, qfd::kTileSmem, s>>>(bva, active, src_base, cw, logR, l0, tiles);
+  });
+}
+// The same from an element vector (the block-folded table).
+static void copy_mobius(cudaStream_t s, const Fe* src, Fe* cw, int logR, int logm) {
+  check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
+  const int l0 = first_mobius_levels(logm, logR);
+  const uint64_t n = uint64_t(1) << logm;
+#if !defined(QF_FIELD_KB)
+  if (mma_transforms(logm, logR)) {
+    qfd::TcPass p = tile_pass(src, cw, logR, logm);
+    launch(s, true, "k_transform_copy_mobius", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0), [&] { CopyMobius::run(s, p); });
+    return;
+  }
+#endif
+  const uint32_t tiles = uint32_t(n >> l0);
+  launch(s, true, "k_copy_mobius_tile", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, l0, 1, 0), [&] {
+    qfd::k_copy_mobius_tile<<<tile_grid(tiles), qfd::kTileThreads, qfd::kTileSmem, s>>>(src, cw, logR, l0, tiles);
+  });
 }
 
 // Inner levels of a row tree over the n_leaves digests at tree[0..): level j
@@ -648,6 +862,7 @@ void GpuBackend::encode_and_hash(DeviceCodeword& out, const Fe* alpha, int logR,
   uint4 r[2];
   QF_CK(cudaMemcpyAsync(r, out.tree.p + 2 * out.level_off.back(), 32, cudaMemcpyDeviceToHost, s_));
   QF_CK(cudaStreamSynchronize(s_));
+  check_transforms();
   out.root_ = digest_from_words(r);
 }
 
@@ -701,6 +916,7 @@ bool DeviceSetup::encode_level(const QaCode<F>& target, const QaCode<F>& current
     QF_CK(cudaMemcpyAsync(encoded.data(), cw.p, er * hc * 16, cudaMemcpyDeviceToHost, s));
     QF_CK(cudaMemcpyAsync(leaves.data(), lv.p, er * 32, cudaMemcpyDeviceToHost, s));
     QF_CK(cudaStreamSynchronize(s));
+    check_transforms();
   }
   QF_CK(cudaStreamDestroy(s));
   return true;
@@ -719,14 +935,8 @@ static std::unique_ptr<DeviceCodeword> alloc_codeword(size_t R, size_t cols, cud
 Digest GpuBackend::encode_block(const W* bva, uint64_t active, uint64_t src_base, DeviceCodeword& cw) {
   const int logm = ilog2(P_.pcs.packed_len());
   const int logR = logm - ilog2(P_.pcs.pp->extension_columns);
-  const int l0 = std::min(qfd::kMaxTileLog, logm);
-  const size_t smem = qfd::kTileSmem;
-  check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
-  QF_LAUNCH_OPS(s_, "k_pack_mobius_tile", (uint64_t(1) << logm) * (F::kLanes * sizeof(W) + 16),
-            qf_intops::transform_ops(kOps, uint64_t(1) << logm, 0, l0, 1, 0),
-            qfd::k_pack_mobius_tile<<<tile_grid(uint64_t(1) << (logm - l0)), qfd::kTileThreads, smem, s_>>>(
-                bva, active, src_base, cw.cw.p, logR, l0, uint32_t(uint64_t(1) << (logm - l0))));
-  encode_and_hash(cw, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, l0);
+  pack_mobius(s_, true, bva, active, src_base, cw.cw.p, logR, logm);
+  encode_and_hash(cw, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, first_mobius_levels(logm, logR));
   return cw.root_;
 }
 
@@ -790,13 +1000,9 @@ void commit_block_into(const Parameters<F>& P, const W* d_bva, uint64_t active, 
   const int logR = logm - ilog2(cols);
   const size_t R = size_t(1) << logR;
   check(P.pcs.pp->seq.top().message_len == R, "alpha table length");
-  // Message half: pack + Mobius levels 0..11, then the rest of the encode.
-  const int l0 = std::min(qfd::kMaxTileLog, logm);
-  check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
-  qfd::k_pack_mobius_tile<<<tile_grid(uint64_t(1) << (logm - l0)), qfd::kTileThreads, qfd::kTileSmem, s>>>(
-      d_bva, active, uint64_t(b) * P.block_len, cw, logR, l0, uint32_t(uint64_t(1) << (logm - l0)));
-  QF_CK(cudaGetLastError());
-  encode_passes(s, cw, alpha, logR, logm, l0, false, false);
+  // Message half: pack + the first Mobius levels, then the rest of the encode.
+  pack_mobius(s, false, d_bva, active, uint64_t(b) * P.block_len, cw, logR, logm);
+  encode_passes(s, cw, alpha, logR, logm, first_mobius_levels(logm, logR), false, false);
   // Row leaves, inner levels, root.
   const uint64_t n_ext = 2 * R;
   qfd::k_hash_leaves<11><<<unsigned((n_ext + qfd::kLeafThreads - 1) / qfd::kLeafThreads), qfd::kLeafThreads, 0, s>>>(
@@ -1060,13 +1266,8 @@ Digest GpuBackend::fold_and_commit(const std::vector<F>& fw) {
     block_fold_launch(bva_, active_, blocks, dT.p, 0);
   }
   folded_ = alloc_codeword(size_t(1) << logR, P_.pcs.pp->extension_columns, s_);
-  const int l0 = std::min(qfd::kMaxTileLog, logm);
-  const size_t smem = qfd::kTileSmem;
-  check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
-  QF_LAUNCH_OPS(s_, "k_copy_mobius_tile", (uint64_t(2) << logm) * 16,
-                qf_intops::transform_ops(kOps, uint64_t(1) << logm, 0, l0, 1, 0), qfd::k_copy_mobius_tile<<<tile_grid(uint64_t(1) << (logm - l0)), qfd::kTileThreads, smem, s_>>>(
-                values_.p, folded_->cw.p, logR, l0, uint32_t(uint64_t(1) << (logm - l0))));
-  encode_and_hash(*folded_, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, l0);
+  copy_mobius(s_, values_.p, folded_->cw.p, logR, logm);
+  encode_and_hash(*folded_, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, first_mobius_levels(logm, logR));
   host_v_.clear();
   host_w_.clear();
   sum_len_ = m;
@@ -1318,12 +1519,8 @@ Digest GpuBackend::commit_folded_values(const std::vector<F>& values) {
   values_.alloc(m);
   QF_CK(cudaMemcpyAsync(values_.p, values.data(), m * 16, cudaMemcpyHostToDevice, s_));
   folded_ = alloc_codeword(size_t(1) << logR, P_.pcs.pp->extension_columns, s_);
-  const int l0 = std::min(qfd::kMaxTileLog, logm);
-  check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
-  QF_LAUNCH_OPS(s_, "k_copy_mobius_tile", (uint64_t(2) << logm) * 16,
-                qf_intops::transform_ops(kOps, uint64_t(1) << logm, 0, l0, 1, 0), qfd::k_copy_mobius_tile<<<tile_grid(uint64_t(1) << (logm - l0)), qfd::kTileThreads, qfd::kTileSmem, s_>>>(
-                values_.p, folded_->cw.p, logR, l0, uint32_t(uint64_t(1) << (logm - l0))));
-  encode_and_hash(*folded_, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, l0);
+  copy_mobius(s_, values_.p, folded_->cw.p, logR, logm);
+  encode_and_hash(*folded_, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, first_mobius_levels(logm, logR));
   QF_CK(cudaStreamSynchronize(s_));  // the host copy of `values` may go once this returns
   host_v_.clear();
   host_w_.clear();
