@@ -227,7 +227,9 @@ inline void append_frame(std::vector<uint8_t>& out, const char* label, const voi
   out.insert(out.end(), p, p + len);
 }
 inline void put_u64(std::vector<uint8_t>& out, uint64_t v) {
-  for (int i = 0; i < 8; ++i) out.push_back(uint8_t(v >> (8 * i)));
+  uint8_t b[8];
+  for (int i = 0; i < 8; ++i) b[i] = uint8_t(v >> (8 * i));
+  out.insert(out.end(), b, b + 8);
 }
 inline std::array<uint8_t, 8> le64(uint64_t v) {
   std::array<uint8_t, 8> b;

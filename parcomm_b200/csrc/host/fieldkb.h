@@ -68,14 +68,15 @@ struct Kb4 {
   QF_HD Kb4& operator+=(const Kb4& o) { *this = *this + o; return *this; }
   QF_HD Kb4& operator-=(const Kb4& o) { *this = *this - o; return *this; }
   QF_HD Kb4 operator*(const Kb4& o) const {
-    // Schoolbook with X^4 = 3: each product is reduced to < p first, so a
-    // coefficient sums at most 4 values < p plus 3 times 3 more (< 2^35).
+    // Schoolbook with X^4 = 3, the wrap-around factor taken into o first: a
+    // coefficient is one sum of four products below p^2 < 2^62, reduced once.
+    uint32_t w[4];
+    for (int j = 0; j < 4; ++j) w[j] = kb_add(kb_add(o.c[j], o.c[j]), o.c[j]);
     uint64_t acc[4] = {0, 0, 0, 0};
     for (int i = 0; i < 4; ++i)
       for (int j = 0; j < 4; ++j) {
-        const uint64_t p = kb_mul(c[i], o.c[j]);
         const int k = i + j;
-        if (k < 4) acc[k] += p; else acc[k - 4] += 3u * p;
+        acc[k & 3] += uint64_t(c[i]) * (k < 4 ? o.c[j] : w[j]);
       }
     Kb4 r;
     for (int k = 0; k < 4; ++k) r.c[k] = kb_reduce64(acc[k]);
@@ -112,8 +113,12 @@ struct Kb4 {
 
   static constexpr int kBytes = 16;
   QF_HD void to_bytes(uint8_t out[16]) const {
+#if !defined(__CUDA_ARCH__) && defined(__SSE2__)  // little-endian storage is the wire encoding
+    std::memcpy(out, c, 16);
+#else
     for (int i = 0; i < 4; ++i)
       for (int j = 0; j < 4; ++j) out[4 * i + j] = uint8_t(c[i] >> (8 * j));
+#endif
   }
   static bool from_bytes(const uint8_t in[16], Kb4& out) {
     for (int i = 0; i < 4; ++i) {

@@ -563,6 +563,7 @@ BatchOpening<F> open_single(const PackedPcs<F>& pcs, SingleBackend<F>& be, const
   const std::vector<uint8_t> ob = opening_to_bytes(op.proof);
   const std::vector<uint8_t> db = decide_to_bytes(dp);
   ByteWriter w;
+  w.out.reserve(64 + (2 + evaluations.size() + 2 * rounds.size()) * F::kBytes + ob.size() + db.size());
   w.bytes(F::kPackedMagic, 8);
   w.field(claimed);
   for (const F& v : evaluations) w.field(v);

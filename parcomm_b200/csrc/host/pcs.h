@@ -116,6 +116,11 @@ struct ByteWriter {
   void len(uint64_t v) { put_u64(out, v); }
   void digest(const Digest& d) { bytes(d.data(), 32); }
   template <class F> void field(const F& v) { uint8_t e[F::kBytes]; v.to_bytes(e); bytes(e, F::kBytes); }
+  template <class F> void fields(const std::vector<F>& v) {
+    const size_t at = out.size();
+    out.resize(at + v.size() * F::kBytes);
+    for (size_t i = 0; i < v.size(); ++i) v[i].to_bytes(out.data() + at + i * F::kBytes);
+  }
 };
 struct ByteReader {
   const uint8_t* p;
@@ -151,7 +156,7 @@ void write_rows(ByteWriter& w, const Rows<F>& r) {
     w.len(r.partial.size());
     for (const auto& q : r.partial) {
       w.len(q.row.size());
-      for (const F& v : q.row) w.field(v);
+      w.fields(q.row);
       write_path<F>(w, q.path);
     }
   } else {
@@ -159,7 +164,7 @@ void write_rows(ByteWriter& w, const Rows<F>& r) {
     w.len(r.n_rows);
     w.len(r.n_cols);
     w.len(r.encoded.size());
-    for (const F& v : r.encoded) w.field(v);
+    w.fields(r.encoded);
   }
 }
 inline Path read_path(ByteReader& r) {
