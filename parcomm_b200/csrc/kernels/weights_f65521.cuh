@@ -142,9 +142,9 @@ __global__ void __launch_bounds__(kTermThreads) k_project_terms(const int8_t* __
 // thread takes groups of 4 rows, lanes 8 lh .. 8 lh + 7 and coefficients
 // 4 h .. 4 h + 3 (thread 4 g + 2 lh + h).  The 4 rows' weights of a lane and
 // the 4 rows' low (high) bytes of a table coefficient transpose into words,
-// so each dp4a adds 4 products.  A thread sums at most 16 rows of a tile
-// (16 * 128 * 65520 < 2^28), a warp reduce-scatter over the 8 lanes of the
-// same (lh, h) stays below 2^31, then i64 across warps and one reduction.
+// so each dp4a adds 4 products.  A thread sums at most 64 rows of a tile, a
+// warp reduce-scatter the 8 lanes of the same (lh, h), low and high bytes
+// apart (512 * 128 * 255 < 2^24), then i64 across warps and one reduction.
 __global__ void __launch_bounds__(kTermThreads) k_project_terms16(const int8_t* __restrict__ bva, uint64_t active,
                                                                   const TermTiles* __restrict__ terms, int n_terms,
                                                                   uint32_t n_tiles, const Fe* __restrict__ tables,
@@ -216,24 +216,32 @@ __global__ void __launch_bounds__(kTermThreads) k_project_terms16(const int8_t* 
         }
       }
     }
-    int32_t acc[32];
-#pragma unroll
-    for (int f = 0; f < 32; ++f) acc[f] = lo[f >> 2][f & 3] + 256 * hi[f >> 2][f & 3];
     // Reduce-scatter over the 8 lanes with the same (lh, h): the lane keeps
     // entries (lane & 28) .. + 3, i.e. lane 8 lh + ((lane >> 2) & 7),
-    // coefficients 4 h .. 4 h + 3.
+    // coefficients 4 h .. 4 h + 3.  The sums of the low and of the high bytes
+    // stay apart (below 2^24 each): together they can pass 2^31.
+    auto reduce_scatter = [&](int32_t (&t)[8][4]) {
+      int32_t acc[32];
 #pragma unroll
-    for (int o = 16, n = 32; o >= 4; o >>= 1, n >>= 1) {
-      const bool upper = lane & o;
+      for (int f = 0; f < 32; ++f) acc[f] = t[f >> 2][f & 3];
 #pragma unroll
-      for (int qq = 0; qq < n / 2; ++qq) {
-        const int32_t send = upper ? acc[qq] : acc[qq + n / 2];
-        const int32_t keep = upper ? acc[qq + n / 2] : acc[qq];
-        acc[qq] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      for (int o = 16, n = 32; o >= 4; o >>= 1, n >>= 1) {
+        const bool upper = lane & o;
+#pragma unroll
+        for (int qq = 0; qq < n / 2; ++qq) {
+          const int32_t send = upper ? acc[qq] : acc[qq + n / 2];
+          const int32_t keep = upper ? acc[qq + n / 2] : acc[qq];
+          acc[qq] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
       }
-    }
-#pragma unroll
-    for (int qq = 0; qq < 4; ++qq) part_s[warp][8 * lh + ((lane >> 2) & 7)][4 * h + qq] = acc[qq];
+      return make_int4(acc[0], acc[1], acc[2], acc[3]);
+    };
+    const int4 sl = reduce_scatter(lo), sh = reduce_scatter(hi);
+    int64_t* to = &part_s[warp][8 * lh + ((lane >> 2) & 7)][4 * h];
+    to[0] = sl.x + 256 * int64_t(sh.x);
+    to[1] = sl.y + 256 * int64_t(sh.y);
+    to[2] = sl.z + 256 * int64_t(sh.z);
+    to[3] = sl.w + 256 * int64_t(sh.w);
     __syncthreads();
     if (threadIdx.x < 16) {
       int64_t sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
