@@ -64,11 +64,11 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Shared-memory matrix descriptor, 128-byte swizzle: start address, leading
-// and stride byte offsets in 16-byte units, descriptor version 1.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lead, uint32_t stride) {
+// Shared-memory matrix descriptor: start address, leading and stride byte
+// offsets in 16-byte units, descriptor version 1, swizzle (2: 128 bytes, 0: none).
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lead, uint32_t stride, uint32_t swizzle = 2) {
   return uint64_t((addr >> 4) & 0x3fffu) | (uint64_t((lead >> 4) & 0x3fffu) << 16) | (uint64_t((stride >> 4) & 0x3fffu) << 32) |
-         (uint64_t(1) << 46) | (uint64_t(2) << 61);
+         (uint64_t(1) << 46) | (uint64_t(swizzle) << 61);
 }
 // Instruction descriptor of kind::i8: s32 accumulators, A signed and K-major,
 // B unsigned and N-major.
@@ -89,7 +89,7 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// 64 (or 32) consecutive columns of this warp's 32 lanes (one lane per thread), waited
+// 64 (32, 16) consecutive columns of this warp's 32 lanes (one lane per thread), waited
 // for in the same statement so that no use of them can move ahead of the wait.
 __device__ __forceinline__ void tmem_ld64(uint32_t (&v)[64], uint32_t tmem) {
   asm volatile(
@@ -122,6 +122,27 @@ __device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t tmem) {
         "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(tmem)
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t tmem) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(tmem)
+      : "memory");
+}
+
+// Contiguous copy from global to shared memory (both addresses and the size
+// multiples of 16 bytes); the barrier counts its bytes, announced by
+// mbar_expect, which is also the phase's arrival.
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem), "l"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
 }
 
 }  // namespace tc5

@@ -7,6 +7,7 @@
 #include "kernels/dot_mma.cuh"
 #if !defined(QF_FIELD_KB)
 #include "kernels/imma_f65521.cuh"
+#include "kernels/project_mma.cuh"
 #include "kernels/transform_mma.cuh"
 #endif
 #include "intops.h"
@@ -533,7 +534,7 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
 static constexpr int kMmaMinLogm = 23;
 static bool mma_transforms(int logm, int logR) { return logm >= kMmaMinLogm && logR >= qfd::kTcTileLog; }
 
-// A wait that gave up in k_transform: one flag per process in host memory
+// A wait that gave up in a tensor-core kernel: one flag per process in host memory
 // that the device can write.
 static int* transform_error() {
   static int* flag = [] {
@@ -545,7 +546,7 @@ static int* transform_error() {
   return flag;
 }
 static void check_transforms() {
-  if (*static_cast<volatile int*>(transform_error())) fail(QF_E_CUDA, "CUDA: a transform pass gave up waiting");
+  if (*static_cast<volatile int*>(transform_error())) fail(QF_E_CUDA, "CUDA: a tensor-core kernel gave up waiting");
 }
 
 template <int CFG, int SRC, int OP1, int OP2, int MID, bool HASY>
@@ -572,6 +573,7 @@ static void configure_transforms() {
   StridedWht::configure();
   MobiusWht::configure();
   MobiusWhtShort::configure();
+  set_smem(qfd::k_project_terms_mma, qfd::kPmSmem);
 }
 
 // Codeword stride of logical index bit `bit` (message half).
@@ -1650,6 +1652,28 @@ qfd::TermTiles term_tiles(TableBuilder& tb, const std::array<F, 2>* f, size_t nh
   return T;
 }
 uint64_t term_tile_count(const qfd::TermTiles& T) { return (T.rows + (uint64_t(1) << T.lb) - 1) >> T.lb; }
+
+// Numbers the groups of a launch's list (its `n` entries hold `tiles` tiles,
+// over `active` weights) for the tensor-core projection; 0 when the list is
+// not for it: lanes other than 16, or an entry that reaches past the weights
+// or starts off a row of 16 (its rows are copied 16 bytes at a time).
+uint32_t plan_groups(qfd::TermTiles* t, size_t n, uint64_t tiles, uint64_t active, size_t lanes) {
+  uint32_t groups = 0;
+  for (size_t k = 0; k < n; ++k) t[k].tiles = uint32_t((k + 1 < n ? t[k + 1].first_tile : tiles) - t[k].first_tile);
+#if !defined(QF_FIELD_KB)
+  if (lanes != 16) return 0;
+  for (size_t k = 0; k < n; ++k) {
+    const uint64_t rows = std::min<uint64_t>(t[k].rows, (uint64_t(t[k].tile_skip) + t[k].tiles) << t[k].lb);
+    if (t[k].offset % 16 || t[k].offset + rows * 16 > active) return 0;
+    t[k].first_group = groups;
+    groups += qfd::pm_groups(t[k]);
+  }
+#else
+  (void)active;
+  (void)lanes;
+#endif
+  return groups;
+}
 }  // namespace
 
 // Lane projections (tbv.rs:288-352) of large terms: one CTA per tile of up
@@ -1718,6 +1742,7 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
   // outputs block-major too, so a piece's tiles are one segment.
   std::vector<qfd::TermTiles> all;
   std::vector<std::vector<size_t>> piece_at(live, std::vector<size_t>(G));
+  std::vector<std::vector<uint32_t>> groups_bg(live, std::vector<uint32_t>(G, 0));
   std::vector<std::vector<uint64_t>> tile_base(live, std::vector<uint64_t>(G));
   std::vector<uint64_t> tiles_g(G, 0);
   std::vector<std::vector<uint32_t>> seg(G, std::vector<uint32_t>(1, 0));
@@ -1726,6 +1751,8 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
     for (size_t g = 0; g < G; ++g) {
       piece_at[b][g] = all.size();
       tile_base[b][g] = tiles_g[g];
+      groups_bg[b][g] = plan_groups(pieces[b][g].data(), pieces[b][g].size(), tiles_bg[b][g],
+                                    std::min<uint64_t>(bl, active_ - uint64_t(b) * bl), lanes_of[g]);
       for (size_t k = 0; k < pieces[b][g].size(); ++k) {
         all.push_back(pieces[b][g][k]);
         const uint64_t end = k + 1 < pieces[b][g].size() ? pieces[b][g][k + 1].first_tile : tiles_bg[b][g];
@@ -1743,7 +1770,7 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
     for (size_t g = 0; g < G; ++g) {
       const uint64_t tiles = tiles_bg[b][g];
       if (!tiles) continue;
-      project_terms_launch(d, n, dall.p + piece_at[b][g], int(pieces[b][g].size()), tiles, tables.p, lanes_of[g],
+      project_terms_launch(d, n, dall.p + piece_at[b][g], int(pieces[b][g].size()), tiles, groups_bg[b][g], tables.p, lanes_of[g],
                            dtile[g].p + tile_base[b][g] * lanes_of[g], n * sizeof(W));
     }
   });
@@ -1758,24 +1785,35 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
     std::vector<F> h(np * lanes_of[g]);
     QF_CK(cudaMemcpyAsync(h.data(), dpiece.p, h.size() * 16, cudaMemcpyDeviceToHost, s_));
     QF_CK(cudaStreamSynchronize(s_));
+    check_transforms();
     for (size_t k = 0; k < np; ++k)
       for (size_t l = 0; l < lanes_of[g]; ++l) out[g][seg_term[g][k]][l] += h[k * lanes_of[g] + l];
   }
   return out;
 }
 
-// Lane projections of `n_terms` term tile lists (`tiles` tiles) into out:
-// the dp4a kernel for F65521 terms of 16 lanes, the general one otherwise.
+// Lane projections of `n_terms` term tile lists (`tiles` tiles) into out.
+// F65521 terms of 16 lanes: on the tensor cores when the list has `groups`
+// (plan_groups) and the weights are 16-byte aligned (HBM-bound), else the dp4a
+// kernel; other lane widths and KoalaBear: the general one.
 void GpuBackend::project_terms_launch(const W* bva, uint64_t active, const qfd::TermTiles* terms, int n_terms,
-                                      uint64_t tiles, const Fe* tables, size_t lanes, Fe* out, uint64_t bytes) {
+                                      uint64_t tiles, uint32_t groups, const Fe* tables, size_t lanes, Fe* out, uint64_t bytes) {
   const unsigned grid = unsigned((tiles + qfd::kTilesPerCta - 1) / qfd::kTilesPerCta);
 #if !defined(QF_FIELD_KB)
+  if (groups && reinterpret_cast<uintptr_t>(bva) % 16 == 0) {
+    QF_LAUNCH(s_, "k_project_terms", bytes,
+              qfd::k_project_terms_mma<<<tile_grid(groups), qfd::kPmThreads, qfd::kPmSmem, s_>>>(bva, terms, n_terms, groups, tables, out,
+                                                                                           transform_error()));
+    return;
+  }
   if (lanes == 16) {
     QF_LAUNCH(s_, "k_project_terms", bytes,
               qfd::k_project_terms16<<<grid, qfd::kTermThreads, 0, s_>>>(bva, active, terms, n_terms, uint32_t(tiles),
                                                                          tables, out));
     return;
   }
+#else
+  (void)groups;
 #endif
   QF_LAUNCH(s_, "k_project_terms", bytes,
             qfd::k_project_terms<<<grid, qfd::kTermThreads, 0, s_>>>(bva, active, terms, n_terms, uint32_t(tiles), tables,
@@ -1820,21 +1858,27 @@ std::vector<std::vector<F>> GpuBackend::project_terms(const std::vector<const Te
     // One launch per term (a bucket's claim term, or a padding / suffix
     // term): each term's tiles renumbered from 0, its outputs at its first tile.
     std::vector<qfd::TermTiles> solo = tt;
-    for (auto& T : solo) T.first_tile = 0;
+    std::vector<uint32_t> groups;
+    for (auto& T : solo) {
+      T.first_tile = 0;
+      groups.push_back(plan_groups(&T, 1, term_tile_count(T), active_, common_lanes));
+    }
     QF_CK(cudaMemcpyAsync(dtt.p, solo.data(), solo.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
     for (size_t k = 0; k < tt.size(); ++k) {
       const uint64_t n = term_tile_count(tt[k]);
-      project_terms_launch(bva_, active_, dtt.p + k, 1, n, tables.p, common_lanes,
+      project_terms_launch(bva_, active_, dtt.p + k, 1, n, groups[k], tables.p, common_lanes,
                            dtile.p + size_t(tt[k].first_tile) * common_lanes, tt[k].rows * common_lanes * sizeof(W) + n * 16);
     }
   } else {
+    const uint32_t groups = plan_groups(tt.data(), tt.size(), tiles, active_, common_lanes);
     QF_CK(cudaMemcpyAsync(dtt.p, tt.data(), tt.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
-    project_terms_launch(bva_, active_, dtt.p, int(tt.size()), tiles, tables.p, common_lanes, dtile.p, proj_bytes);
+    project_terms_launch(bva_, active_, dtt.p, int(tt.size()), tiles, groups, tables.p, common_lanes, dtile.p, proj_bytes);
   }
   QF_LAUNCH(s_, "k_sum_segments", tiles * common_lanes * 16, qfd::k_sum_segments<<<unsigned(terms.size()), kThreads, 0, s_>>>(dtile.p, dseg.p, int(common_lanes), dterm.p));
   std::vector<F> h(terms.size() * common_lanes);
   QF_CK(cudaMemcpyAsync(h.data(), dterm.p, h.size() * 16, cudaMemcpyDeviceToHost, s_));
   QF_CK(cudaStreamSynchronize(s_));
+  check_transforms();
   for (size_t t = 0; t < terms.size(); ++t)
     for (size_t l = 0; l < common_lanes; ++l) out[t][l] = h[t * common_lanes + l];
   return out;

@@ -118,6 +118,7 @@ struct TermTiles {
   uint32_t tile_skip;  // the term's tiles before the first one of this list entry (0 unless a term is split)
   uint32_t lo_off, mid_off, top_off;
   uint32_t lb, mb;
+  uint32_t tiles, first_group;  // tiles of this list entry, and its first group of eight (tensor-core projection)
 };
 __device__ __forceinline__ int find_term(const TermTiles* __restrict__ t, int n, uint32_t tile) {
   int lo = 0, hi = n - 1;
