@@ -90,35 +90,47 @@ __device__ __forceinline__ void audit_group(Frac& f, const AlphaPowers& ap, cons
   // at most three of them and two canonical terms in one 64-bit sum; F65521:
   // products below 2^35).
   uint32_t m[G];
+  Fr P, D;
+#if !defined(QF_FIELD_KB)
 #pragma unroll
   for (int k = 0; k < G; ++k) m[k] = red_signed(c[k]);
-  Fr P, D;
 #pragma unroll
   for (int j = 0; j < kC; ++j) {
     uint64_t s = ap.c[G - 1][j], t;
-    if constexpr (sizeof(Wt) == 1) {
-      t = uint64_t(G) * ap.c[G - 2][j];
+    t = uint64_t(G) * ap.c[G - 2][j];
 #pragma unroll
-      for (int k = 1; k < G; ++k) s += uint64_t(m[k]) * ap.c[k - 1][j];
+    for (int k = 1; k < G; ++k) s += uint64_t(m[k]) * ap.c[k - 1][j];
 #pragma unroll
-      for (int k = 2; k < G; ++k) t += uint64_t(k * m[k]) * ap.c[k - 2][j];
-      if (j == 0) { s += m[0]; t += m[1]; }
-      P.c[j] = red_sum(s);
-      D.c[j] = red_sum(t);
-    } else {
-      // G = 4: P = a^4 + m3 a^3 + m2 a^2 + m1 a + m0, P' = 4 a^3 + 3 m3 a^2 + 2 m2 a + m1.
-      s += uint64_t(m[3]) * ap.c[2][j] + uint64_t(m[2]) * ap.c[1][j] + uint64_t(m[1]) * ap.c[0][j];
-      t = 4ull * ap.c[2][j] + uint64_t(red_signed(3 * c[3])) * ap.c[1][j] + uint64_t(red_signed(2 * c[2])) * ap.c[0][j];
-      if (j == 0) { s += m[0]; t += m[1]; }
-      P.c[j] = red_sum(s);
-      D.c[j] = red_sum(t);
-    }
+    for (int k = 2; k < G; ++k) t += uint64_t(k * m[k]) * ap.c[k - 2][j];
+    if (j == 0) { s += m[0]; t += m[1]; }
+    P.c[j] = red_sum(s);
+    D.c[j] = red_sum(t);
   }
   Acc t = acc_zero();
   mul_acc(t, f.n, P);
   mul_acc(t, D, f.d);
   f.n = acc_reduce(t);
   f.d = mul(f.d, P);
+#else
+  // G = 4: P = a^4 + m3 a^3 + m2 a^2 + m1 a + m0, P' = 4 a^3 + 3 m3 a^2 + 2 m2
+  // a + m1.  Only the ratio n / d counts, so every product keeps the 2^-32 of
+  // its Montgomery reduction: P and P' carry the same power (the m_k bring
+  // one, the terms without an m_k are given it), and so do n and d after.
+#pragma unroll
+  for (int k = 0; k < G; ++k) m[k] = redc(uint64_t(c[k] + (long long)kBias));
+  const uint32_t m3 = addp(addp(m[3], m[3]), m[3]), m2 = addp(m[2], m[2]);
+#pragma unroll
+  for (int j = 0; j < kC; ++j) {
+    uint64_t s = redc(ap.c[3][j]), t = redc(4ull * ap.c[2][j]);  // loop invariants
+    s += uint64_t(m[3]) * ap.c[2][j] + uint64_t(m[2]) * ap.c[1][j] + uint64_t(m[1]) * ap.c[0][j];
+    t += uint64_t(m3) * ap.c[1][j] + uint64_t(m2) * ap.c[0][j];
+    if (j == 0) { s += m[0]; t += m[1]; }
+    P.c[j] = redc(s);
+    D.c[j] = redc(t);
+  }
+  f.n = add(mul_redc(f.n, P), mul_redc(f.d, D));
+  f.d = mul_redc(f.d, P);
+#endif
 }
 
 // n / d += 1 / (alpha - v).
