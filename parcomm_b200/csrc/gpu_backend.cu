@@ -808,11 +808,11 @@ static void copy_mobius(cudaStream_t s, const Fe* src, Fe* cw, int logR, int log
 }
 
 // Inner levels of a row tree over the n_leaves digests at tree[0..): level j
-// at digest offset level_off[j], the root last.  Launches of two levels per
-// thread (k_hash_subtrees: each thread hashes a 4-child subtree, no barrier;
-// three levels measured slower, their registers cost occupancy) while the
-// level they reach keeps at least 2^11 nodes, then one CTA for the levels
-// above (k_hash_top): 7 launches for 2^23 leaves instead of 23.
+// at digest offset level_off[j], the root last; the digest after it is spare.
+// Launches of two levels per thread (k_hash_subtrees: each thread hashes a
+// 4-child subtree, no barrier; three levels measured slower, their registers
+// cost occupancy) while the level they reach keeps at least 2^16 nodes, then
+// one launch for the levels above (k_hash_top): 5 launches for 2^23 leaves.
 static void build_tree(cudaStream_t s, uint4* tree, uint64_t n_leaves, std::vector<uint64_t>& level_off, bool timed) {
   level_off.clear();
   for (uint64_t k = n_leaves, off = 0;; k /= 2) {
@@ -821,7 +821,7 @@ static void build_tree(cudaStream_t s, uint4* tree, uint64_t n_leaves, std::vect
     if (k <= 1) break;
   }
   const ::qfd::InnerPrefix ip = inner_prefix();
-  constexpr int kTopLog = 11;
+  constexpr int kTopLog = qfd::kTopLog;
   size_t j = 0;
   uint64_t n = n_leaves;
   while (n > (uint64_t(1) << kTopLog)) {
@@ -841,7 +841,10 @@ static void build_tree(cudaStream_t s, uint4* tree, uint64_t n_leaves, std::vect
     qfd::TreeLevels lv{};
     for (int t = 0; t <= ilog2(n); ++t) lv.off[t] = level_off[j + t];
     launch(s, timed, "k_hash_inner", n * 32 + (n - 1) * 32, qf_intops::inner_hash_ops(n - 1),
-           [&] { qfd::k_hash_top<<<1, unsigned(std::min<uint64_t>(1024, n / 2)), 0, s>>>(tree, n, lv, ip); });
+           [&] {
+             qfd::k_hash_top<<<unsigned((n + qfd::kTopChildren - 1) / qfd::kTopChildren), qfd::kTopThreads, 0, s>>>(
+                 tree, n, lv, ip, reinterpret_cast<unsigned int*>(tree + 2 * (2 * n_leaves - 1)));
+           });
   }
 }
 

@@ -829,52 +829,59 @@ __global__ void k_hash_setup_rows(const Fe* __restrict__ cw, uint64_t n_rows, in
   leaves[2 * row + 1] = make_uint4(h[4], h[5], h[6], h[7]);
 }
 
-constexpr int kLeafThreads = 64;
-constexpr int kRowWords = 128;  // 32 entries x 4 words
-constexpr int kRowStride = 129;  // padded: conflict-free per-thread rows
-
-// TAIL = prefix bytes after the 64-byte midstate: 11 for the 75-byte
-// base-row prefix, 16 for the 80-byte extension-row prefix.
+// Row leaves, one thread per row: BLAKE2s of the prefix's tail (its first 64
+// bytes are in the midstate) and the row's n_cols elements.  TAIL = prefix
+// bytes after the midstate: 11 for the 75-byte base-row prefix, 16 for the
+// 80-byte extension-row prefix.  Each 64-byte block takes four new elements
+// behind what the tail's length leaves over of the four before, all in
+// registers: consecutive threads read consecutive rows of a column, so the
+// loads are whole 512-byte lines without staging, and the next block's are
+// on their way during a compression.  Bound by the ALU pipe (XORs and
+// rotations, 640 a compression).
+constexpr int kLeafThreads = 128;
 template <int TAIL>
 __global__ void __launch_bounds__(kLeafThreads) k_hash_leaves(const Fe* __restrict__ cw, uint64_t n_rows, int n_cols,
                                                               ::qfd::LeafPrefix pre, uint4* __restrict__ leaves) {
   static_assert(TAIL == 11 || TAIL == 16, "leaf prefix");
-  __shared__ uint32_t rows_s[kLeafThreads * kRowStride];
+  constexpr int kKeep = TAIL == 11 ? 3 : 4;  // words left over of a block's sixteen new ones
   const uint64_t r = uint64_t(blockIdx.x) * kLeafThreads + threadIdx.x;
-  uint32_t* mine = rows_s + threadIdx.x * kRowStride;
-  if (r < n_rows) {
-    for (int c = 0; c < n_cols; ++c) {
-      uint4 u = *reinterpret_cast<const uint4*>(cw + size_t(c) * n_rows + r);
-      mine[4 * c] = u.x; mine[4 * c + 1] = u.y; mine[4 * c + 2] = u.z; mine[4 * c + 3] = u.w;
-    }
-  }
   if (r >= n_rows) return;
-  const int nw = 4 * n_cols;  // row words
-  auto rw = [&](int q) -> uint32_t { return q < nw ? mine[q] : 0u; };
+  // The tree's spare digest, behind its 2 n_rows - 1: the ticket of k_hash_top.
+  if (r == 0) leaves[2 * (2 * n_rows - 1)] = make_uint4(0, 0, 0, 0);
+  const uint4* col = reinterpret_cast<const uint4*>(cw) + r;
+  auto fetch = [&](int c, uint4 (&e)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = c + i < n_cols ? __ldg(col + uint64_t(c + i) * n_rows) : make_uint4(0, 0, 0, 0);
+  };
   uint32_t h[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) h[i] = pre.mid[i];
-  // Stream after the midstate: TAIL prefix bytes then the row; 64-byte blocks.
-  const uint32_t total = 64u + TAIL + uint32_t(nw) * 4u;
+  const uint32_t total = 64u + TAIL + uint32_t(n_cols) * 16u;
   const int nblocks = int((total - 64 + 63) / 64);
+  uint32_t x[kKeep + 16];  // the words kept, then the new ones
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) x[i] = TAIL == 16 ? pre.tail[i] : 0u;
+  uint4 e[4];
+  fetch(0, e);
   for (int j = 1; j <= nblocks; ++j) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[kKeep + 4 * i] = e[i].x;
+      x[kKeep + 4 * i + 1] = e[i].y;
+      x[kKeep + 4 * i + 2] = e[i].z;
+      x[kKeep + 4 * i + 3] = e[i].w;
+    }
+    fetch(4 * j, e);
     uint32_t m[16];
 #pragma unroll
-    for (int w = 0; w < 16; ++w) {
-      const int s = 64 * (j - 1) + 4 * w;
-      uint32_t word;
-      if (TAIL == 16) {
-        word = s < 16 ? pre.tail[w] : rw((s - 16) >> 2);
-      } else if (s < 8) {
-        word = pre.tail[w];
-      } else if (s == 8) {
-        word = __byte_perm(pre.tail[2], rw(0), 0x4210);  // pre.tail[2] (3 bytes) | (rw(0) << 24)
-      } else {
-        const int q = (s - 12) >> 2;
-        word = __byte_perm(rw(q), rw(q + 1), 0x4321);  // (rw(q) >> 8) | (rw(q + 1) << 24)
-      }
-      m[w] = word;
+    for (int w = 0; w < 16; ++w) m[w] = TAIL == 16 ? x[w] : __byte_perm(x[w], x[w + 1], 0x4321);  // (x[w] >> 8) | (x[w + 1] << 24)
+    if (TAIL == 11 && j == 1) {
+      m[0] = pre.tail[0];
+      m[1] = pre.tail[1];
+      m[2] = __byte_perm(pre.tail[2], x[3], 0x4210);  // three bytes of tail | (x[3] << 24)
     }
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) x[i] = x[16 + i];
     const bool last = j == nblocks;
     ::qfd::compress(h, m, last ? total : 64u + 64u * uint32_t(j), last, pre.one);
   }
@@ -906,7 +913,7 @@ __device__ __forceinline__ void inner_hash(const uint32_t (&d)[16], const ::qfd:
 // Digest offsets (in digests, 2 uint4 each) of the levels a launch reads and
 // writes: off[0] the children's level, off[j] the level j above it.
 struct TreeLevels {
-  uint64_t off[12];
+  uint64_t off[18];
 };
 
 // The node at height D above level 0 with index `idx` in its level, from its
@@ -943,25 +950,80 @@ __global__ void k_hash_subtrees(uint4* __restrict__ tree, uint64_t n_top, TreeLe
   subtree_hash<L>(tree, lv, i, pre, h);
 }
 
-// The top of a tree in one CTA: from the n children at level off[0] (n a
-// power of two, n / 2 <= blockDim.x) every level up to the root, one node per
-// thread and level, a barrier between levels (the children a level reads are
-// the previous level's stores of other threads of this CTA).
-__global__ void k_hash_top(uint4* __restrict__ tree, uint64_t n, TreeLevels lv, ::qfd::InnerPrefix pre) {
+// inner_hash with one copy of the compression (18 KB of straight-line code):
+// where few warps run, fetching the second copy costs more than the loop.
+__device__ __forceinline__ void inner_hash_rolled(const uint32_t (&d)[16], const ::qfd::InnerPrefix& pre, uint32_t (&h)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) h[k] = ::qfd::kIv[k];
+  h[0] ^= 0x01010020u;
+#pragma unroll 1
+  for (int block = 0; block < 2; ++block) {
+    uint32_t m[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      // Word k of a block: prefix, then the children's words two bytes late.
+      auto late = [&](int q) { return (q == 0 ? pre.w[12] : d[q - 1] >> 16) | (q < 16 ? d[q] << 16 : 0u); };
+      const uint32_t first = k < 12 ? pre.w[k] : late(k - 12), second = k < 13 ? late(k + 4) : 0u;
+      m[k] = block ? second : first;
+    }
+    ::qfd::compress(h, m, block ? 114u : 64u, block != 0, pre.one);
+  }
+}
+
+// The top of a tree in one launch: from the n children at level off[0] (a
+// power of two, at most 2^16) up to the root.  A CTA hashes the subtree over
+// 2 blockDim.x of them, a level at a time through shared memory; the last CTA
+// to finish (a ticket in *done, zeroed by k_hash_leaves) takes the subtrees'
+// roots on to the tree's.  What bounds it is the chain of two compressions a
+// level, which one warp per scheduler already takes at the ALU pipe's rate.
+constexpr int kTopThreads = 128, kTopChildren = 2 * kTopThreads, kTopLog = 16;
+__global__ void __launch_bounds__(kTopThreads) k_hash_top(uint4* tree, uint64_t n, TreeLevels lv, ::qfd::InnerPrefix pre,
+                                                          unsigned int* done) {
+  __shared__ uint4 level_s[2 * kTopThreads];
+  __shared__ unsigned int ticket_s;
+  const uint32_t t = threadIdx.x;
+  uint32_t children = uint32_t(n < kTopChildren ? n : kTopChildren);
+  uint64_t first = uint64_t(blockIdx.x) * children;
   int j = 0;
-  for (uint64_t parents = n / 2; parents >= 1; parents /= 2, ++j) {
-    for (uint64_t i = threadIdx.x; i < parents; i += blockDim.x) {
-      const uint4* c = tree + 2 * (lv.off[j] + 2 * i);
-      uint32_t d[16];
-      const uint4 a = __ldcg(c), b = __ldcg(c + 1), e = __ldcg(c + 2), f = __ldcg(c + 3);
-      d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w; d[4] = b.x; d[5] = b.y; d[6] = b.z; d[7] = b.w;
-      d[8] = e.x; d[9] = e.y; d[10] = e.z; d[11] = e.w; d[12] = f.x; d[13] = f.y; d[14] = f.z; d[15] = f.w;
+  bool top = false;
+#pragma unroll 1
+  for (uint32_t parents = children / 2;;) {
+    if (parents == 0) {  // the subtree's root is done
+      if (gridDim.x == 1 || top) return;
+      top = true;
+      if (t == 0) {  // this thread wrote it
+        __threadfence();
+        ticket_s = atomicAdd(done, 1u);
+      }
+      __syncthreads();
+      if (ticket_s != gridDim.x - 1) return;
+      __threadfence();
+      children = gridDim.x;
+      parents = children / 2;
+      first = 0;
+    }
+    uint4 a, b, e, f;
+    if (t < parents) {
+      if (parents == children / 2) {
+        const uint4* c = tree + 2 * (lv.off[j] + first + 2 * t);
+        a = __ldcg(c), b = __ldcg(c + 1), e = __ldcg(c + 2), f = __ldcg(c + 3);
+      } else {
+        a = level_s[4 * t], b = level_s[4 * t + 1], e = level_s[4 * t + 2], f = level_s[4 * t + 3];
+      }
+    }
+    __syncthreads();  // every child of this level has been read
+    first /= 2;
+    ++j;
+    if (t < parents) {
+      const uint32_t d[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
       uint32_t h[8];
-      inner_hash(d, pre, h);
-      tree[2 * (lv.off[j + 1] + i)] = make_uint4(h[0], h[1], h[2], h[3]);
-      tree[2 * (lv.off[j + 1] + i) + 1] = make_uint4(h[4], h[5], h[6], h[7]);
+      inner_hash_rolled(d, pre, h);
+      uint4* out = tree + 2 * (lv.off[j] + first + t);
+      out[0] = level_s[2 * t] = make_uint4(h[0], h[1], h[2], h[3]);
+      out[1] = level_s[2 * t + 1] = make_uint4(h[4], h[5], h[6], h[7]);
     }
     __syncthreads();
+    parents /= 2;
   }
 }
 
