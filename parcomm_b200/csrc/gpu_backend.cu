@@ -383,9 +383,18 @@ static void wht_tile_launch(cudaStream_t s, const Fe* src, Fe* dst, const Fe* al
     qfd::k_wht_tile<false><<<tile_grid(tiles), qfd::kTileThreads, qfd::kTileSmem, s>>>(src, dst, nullptr, logR, wl, tiles);
 }
 
+// Codewords of fewer than 2^19 message entries have fewer 4096-element tiles
+// than the chip has SMs, and a pass takes as long as one tile: their tiles
+// shrink to 1/128 of the message, 64 elements at least.
+static int small_tile_log(int logm) { return std::max(6, std::min(qfd::kMaxTileLog, logm - 7)); }
+
 // 2^cb consecutive group bases per tile of a k-level strided pass: 64-byte
-// runs at k = 10, the full 4096-element tile below that.
-static int strided_cb(int k, int logm) { return std::min(k >= 10 ? 2 : qfd::kMaxTileLog - k, logm - k); }
+// runs at k = 10, the full 4096-element tile below that (small messages: as
+// above, runs of at least 64 bytes).
+static int strided_cb(int k, int logm) {
+  const int cb = std::min(k >= 10 ? 2 : qfd::kMaxTileLog - k, logm - k);
+  return std::min(cb, std::max(2, small_tile_log(logm) - k));
+}
 
 // ---------------------------------------------------------------- pass autotuner
 // How many levels each strided pass takes is a choice: one deep pass is
@@ -723,7 +732,6 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
   }
 #endif
   constexpr int kT = qfd::kMaxTileLog;
-  check(!mobius || mob_from == kT, "the Mobius tile pass covers bits 0..11");
   const int top = std::min(logR, kT + 10);  // fused span [kT, top)
   const int k = top - kT;
   // KoalaBear does not fuse the Mobius and WHT #1 strided levels: its
@@ -736,7 +744,8 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
 #else
   const bool fused = mobius && k >= 6;
 #endif
-  if (mobius) strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, fused ? top : kT, logm, timed, allow_tuning);
+  check(!fused || mob_from == kT, "the Mobius tile pass covers bits 0..11");
+  if (mobius) strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, fused ? top : mob_from, logm, timed, allow_tuning);
   if (fused) {
     const int cb = strided_cb(k, logm);
     const uint32_t tiles = uint32_t(uint64_t(1) << (logm - k - cb));
@@ -767,7 +776,7 @@ static int first_mobius_levels(int logm, int logR) {
   if (mma_transforms(logm, logR)) return qfd::kTcTileLog;
 #endif
   (void)logR;
-  return std::min(qfd::kMaxTileLog, logm);
+  return std::min(small_tile_log(logm), logm);
 }
 // Packed weights of one block (from entry src_base of the `active` at bva)
 // with their first Mobius levels into the message half at cw.
@@ -855,14 +864,14 @@ void GpuBackend::encode_and_hash(DeviceCodeword& out, const Fe* alpha, int logR,
   // Leaves and inner levels.
   const uint64_t n_ext = 2 * R;
   ::qfd::LeafPrefix lp = leaf_prefix(out.n_cols, ext_domain);
-  const unsigned lgrid = unsigned((n_ext + qfd::kLeafThreads - 1) / qfd::kLeafThreads);
+  const unsigned lthreads = qfd::leaf_threads(n_ext), lgrid = unsigned((n_ext + lthreads - 1) / lthreads);
   const uint64_t leaf_ops = qf_intops::leaf_hash_ops(n_ext, ext_domain ? 80 : 75, out.n_cols * 16);
   if (ext_domain)
     QF_LAUNCH_OPS(s_, "k_hash_leaves", n_ext * out.n_cols * 16 + n_ext * 32, leaf_ops,
-                  qfd::k_hash_leaves<16><<<lgrid, qfd::kLeafThreads, 0, s_>>>(out.cw.p, n_ext, int(out.n_cols), lp, out.tree.p));
+                  qfd::k_hash_leaves<16><<<lgrid, lthreads, 0, s_>>>(out.cw.p, n_ext, int(out.n_cols), lp, out.tree.p));
   else
     QF_LAUNCH_OPS(s_, "k_hash_leaves", n_ext * out.n_cols * 16 + n_ext * 32, leaf_ops,
-                  qfd::k_hash_leaves<11><<<lgrid, qfd::kLeafThreads, 0, s_>>>(out.cw.p, n_ext, int(out.n_cols), lp, out.tree.p));
+                  qfd::k_hash_leaves<11><<<lgrid, lthreads, 0, s_>>>(out.cw.p, n_ext, int(out.n_cols), lp, out.tree.p));
   build_tree(s_, out.tree.p, n_ext, out.level_off, true);
   uint4 r[2];
   QF_CK(cudaMemcpyAsync(r, out.tree.p + 2 * out.level_off.back(), 32, cudaMemcpyDeviceToHost, s_));
@@ -1010,7 +1019,8 @@ void commit_block_into(const Parameters<F>& P, const W* d_bva, uint64_t active, 
   encode_passes(s, cw, alpha, logR, logm, first_mobius_levels(logm, logR), false, false);
   // Row leaves, inner levels, root.
   const uint64_t n_ext = 2 * R;
-  qfd::k_hash_leaves<11><<<unsigned((n_ext + qfd::kLeafThreads - 1) / qfd::kLeafThreads), qfd::kLeafThreads, 0, s>>>(
+  const unsigned lthreads = qfd::leaf_threads(n_ext);
+  qfd::k_hash_leaves<11><<<unsigned((n_ext + lthreads - 1) / lthreads), lthreads, 0, s>>>(
       cw, n_ext, int(cols), leaf_prefix(cols, false), tree);
   QF_CK(cudaGetLastError());
   std::vector<uint64_t> level_off;

@@ -838,13 +838,16 @@ __global__ void k_hash_setup_rows(const Fe* __restrict__ cw, uint64_t n_rows, in
 // loads are whole 512-byte lines without staging, and the next block's are
 // on their way during a compression.  Bound by the ALU pipe (XORs and
 // rotations, 640 a compression).
+// Few rows run one warp per CTA: warps of one SM fetch the straight-line
+// compression separately and slow each other down.
 constexpr int kLeafThreads = 128;
+inline unsigned leaf_threads(uint64_t n_rows) { return n_rows < 148 * kLeafThreads ? 32u : unsigned(kLeafThreads); }
 template <int TAIL>
 __global__ void __launch_bounds__(kLeafThreads) k_hash_leaves(const Fe* __restrict__ cw, uint64_t n_rows, int n_cols,
                                                               ::qfd::LeafPrefix pre, uint4* __restrict__ leaves) {
   static_assert(TAIL == 11 || TAIL == 16, "leaf prefix");
   constexpr int kKeep = TAIL == 11 ? 3 : 4;  // words left over of a block's sixteen new ones
-  const uint64_t r = uint64_t(blockIdx.x) * kLeafThreads + threadIdx.x;
+  const uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (r >= n_rows) return;
   // The tree's spare digest, behind its 2 n_rows - 1: the ticket of k_hash_top.
   if (r == 0) leaves[2 * (2 * n_rows - 1)] = make_uint4(0, 0, 0, 0);
