@@ -530,10 +530,10 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
 // strided passes of six levels or more on the tensor cores
 // (kernels/transform_mma.cuh).  Measured on B200, F65521, against the
 // butterfly kernels, ms per pass:
-//   2^25 entries  WHT of 9 strided levels 0.248 / 0.320, Mobius + WHT 0.500 /
-//                 0.563, WHT alpha WHT 0.731 (13 levels each) / 0.815 (12),
+//   2^25 entries  WHT of 9 strided levels 0.244 / 0.320, Mobius + WHT 0.490 /
+//                 0.563, WHT alpha WHT 0.721 (13 levels each) / 0.815 (12),
 //                 Mobius tile of an element vector 0.223 (13) / 0.309 (12),
-//                 of weights 0.285 (13) / 0.342 (12)
+//                 of weights 0.290 (13) / 0.342 (12)
 //   2^23          0.078 / 0.083, -, 0.203 / 0.213, 0.072 / 0.088, 0.090 / 0.095
 //   2^22          0.053 / 0.045, -, 0.127 / 0.113: 3.5 tiles per SM leave the
 //                 chain of a tile's stages exposed

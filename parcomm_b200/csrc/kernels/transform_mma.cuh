@@ -184,15 +184,14 @@ __device__ __forceinline__ uint32_t tc_next(uint32_t r) { return r + 4 >= NR ? r
 // layout of stage X / Y at unit u0 of chunk 0, 0 leaves it to fin.
 // PARTS 2 takes the columns in two halves, for fewer registers.
 template <int CFG, bool X, int TO, int PARTS, class Before, class Fin>
-__device__ __forceinline__ void tc_chunk(TcBars& B, unsigned char* region, uint32_t tmem, uint32_t u, int c, uint32_t u0, uint32_t c256,
+__device__ __forceinline__ void tc_chunk(TcBars& B, uint32_t region, uint32_t tmem, uint32_t u, int c, uint32_t u0, uint32_t c256,
                                          Before before, Fin fin) {
   using L = TcLayout<CFG, X>;
   using To = TcLayout<CFG, TO == 1>;
   before();
   B.wait(B.full(u & 1), u >> 1);
   tc5::fence_after_sync();
-  uint4* out = reinterpret_cast<uint4*>(region);
-  const uint32_t uc = X ? u0 : u0 ^ uint32_t(c) << 9;  // stage Y's chunk bits, alike in both layouts
+  const uint32_t uc = (X ? u0 : u0 ^ uint32_t(c) << 9) << 4;  // stage Y's chunk bits, alike in both layouts
 #pragma unroll
   for (int h = 0; h < PARTS; ++h) {
     uint32_t d[64 / PARTS];
@@ -211,7 +210,7 @@ __device__ __forceinline__ void tc_chunk(TcBars& B, unsigned char* region, uint3
       for (int j = 0; j < 16; ++j) s[j] = d[16 * q + j];
       Fr v = limb_sums(s, c256);
       fin(i, v);
-      if (TO) out[uc ^ To::unit(L::of_n(i))] = pack_fe(v);
+      if (TO) tc5::store_shared(region + (uc ^ To::unit(L::of_n(i)) << 4), pack_fe(v));
     }
   }
   if (TO) {
@@ -284,16 +283,17 @@ __global__ void __launch_bounds__(tc_threads(SRC), 1) k_transform(const __grid_c
     const uint32_t m = uint32_t(lane) | uint32_t(warp & 3) << 5, g = uint32_t(warp >> 2) << 2;
     const uint32_t ex = LX::of_m(m) | LX::of_n(g), ey = LY::of_m(m) | LY::of_n(g);
     const uint32_t tmem = tmem0 + (uint32_t(warp & 3) << 21) + 16u * g, c256 = p.c256;
+    const uint32_t ring_s = tc5::smem_addr(ring);
     uint32_t u = 0;  // chunks so far
     uint32_t ring_x = 0, ring_y = uint32_t(warp & 3);  // regions of chunk 0, and of this warp's stage Y elements
     auto nothing = [] {};
     auto keep = [](int, Fr&) {};
-    auto x_region = [&](int c) { const uint32_t r = ring_x + c; return ring + (r >= NR ? r - NR : r) * kTcRegionBytes; };
+    auto x_region = [&](int c) { const uint32_t r = ring_x + c; return ring_s + (r >= NR ? r - NR : r) * kTcRegionBytes; };
     auto x_out = [&](Fe* to, int c) { return to + offset(ex) + uint32_t(c & 1) * p.stride[LX::chunk(0)] + uint32_t(c >> 1) * p.stride[LX::chunk(1)]; };
     for (uint32_t vt = blockIdx.x; vt < p.n_tiles; vt += gridDim.x) {
       const uint32_t tile = real_tile(vt);
       const uint32_t tbase = tc_tile_base(p, tile);
-      unsigned char* y_region = ring + ring_y * kTcRegionBytes;
+      const uint32_t y_region = ring_s + ring_y * kTcRegionBytes;
       if constexpr (kTwo && HASY) {
         const uint32_t xy = LY::unit(ex);
 #pragma unroll 1
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(tc_threads(SRC), 1) k_transform(const __grid_c
 #pragma unroll 1
       for (int c = 0; c < 4; ++c, ++u) {
         Fe* dst = x_out(p.dst + tbase, c);
-        tc_chunk<CFG, true, 0, kParts>(B, nullptr, tmem, u, c, 0, c256, nothing, [&](int i, Fr& v) {
+        tc_chunk<CFG, true, 0, kParts>(B, 0, tmem, u, c, 0, c256, nothing, [&](int i, Fr& v) {
           *reinterpret_cast<uint4*>(dst + offset(LX::of_n(i))) = pack_fe(v);
         });
       }
@@ -419,11 +419,11 @@ __global__ void __launch_bounds__(tc_threads(SRC), 1) k_transform(const __grid_c
 #pragma unroll 1
         for (uint32_t c = 0; c < 4; ++c, advance()) {
           if (lap > 0) B.wait(B.unused(r), lap - 1);
-          uint4* to = reinterpret_cast<uint4*>(ring + r * kTcRegionBytes);
+          const uint32_t to = tc5::smem_addr(ring) + r * kTcRegionBytes;
 #pragma unroll
           for (uint32_t i = 0; i < 8; ++i) {
-            to[lu ^ LF::unit(i << 6)] = pack_weights(make_uint2(raw[i].x, raw[i].y));
-            to[lu ^ LF::unit(i << 6 | 1)] = pack_weights(make_uint2(raw[i].z, raw[i].w));
+            tc5::store_shared(to + ((lu ^ LF::unit(i << 6)) << 4), pack_weights(make_uint2(raw[i].x, raw[i].y)));
+            tc5::store_shared(to + ((lu ^ LF::unit(i << 6 | 1)) << 4), pack_weights(make_uint2(raw[i].z, raw[i].w)));
           }
           tc5::mbar_arrive(B.loaded(r));
           if (c < 3) fetch(vt, c + 1);
