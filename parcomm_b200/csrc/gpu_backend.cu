@@ -5,6 +5,7 @@
 #include "kernels/vec.cuh"
 #include "kernels/audit.cuh"
 #include "kernels/dot_mma.cuh"
+#include "kernels/eq_mma.cuh"
 #if !defined(QF_FIELD_KB)
 #include "kernels/imma_f65521.cuh"
 #include "kernels/project_mma.cuh"
@@ -524,6 +525,21 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
   }
 }
 
+// A wait that gave up in a tensor-core kernel: one flag per process in host memory
+// that the device can write.
+static int* transform_error() {
+  static int* flag = [] {
+    int* p = nullptr;
+    QF_CK(cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    *p = 0;
+    return p;
+  }();
+  return flag;
+}
+static void check_transforms() {
+  if (*static_cast<volatile int*>(transform_error())) fail(QF_E_CUDA, "CUDA: a tensor-core kernel gave up waiting");
+}
+
 #if !defined(QF_FIELD_KB)
 // ---------------------------------------------------------------- tensor-core transform passes
 // Codewords of at least 2^23 message entries run their tile passes and the
@@ -542,21 +558,6 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
 // as many coefficients (0.26, 0.45, 0.59 at 2^25): it keeps them.
 static constexpr int kMmaMinLogm = 23;
 static bool mma_transforms(int logm, int logR) { return logm >= kMmaMinLogm && logR >= qfd::kTcTileLog; }
-
-// A wait that gave up in a tensor-core kernel: one flag per process in host memory
-// that the device can write.
-static int* transform_error() {
-  static int* flag = [] {
-    int* p = nullptr;
-    QF_CK(cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
-    *p = 0;
-    return p;
-  }();
-  return flag;
-}
-static void check_transforms() {
-  if (*static_cast<volatile int*>(transform_error())) fail(QF_E_CUDA, "CUDA: a tensor-core kernel gave up waiting");
-}
 
 template <int CFG, int SRC, int OP1, int OP2, int MID, bool HASY>
 struct Transform {
@@ -583,6 +584,7 @@ static void configure_transforms() {
   MobiusWht::configure();
   MobiusWhtShort::configure();
   set_smem(qfd::k_project_terms_mma, qfd::kPmSmem);
+  set_smem(qfd::k_eq_project_tc, qfd::kEtSmem);
 }
 
 // Codeword stride of logical index bit `bit` (message half).
@@ -638,8 +640,10 @@ static qfd::TcPass strided_pass(const void* src, Fe* dst, int logR, int logm, in
   return p;
 }
 #else
-static void configure_transforms() {}
-static void check_transforms() {}
+static void configure_transforms() {
+  transform_error();
+  set_smem(qfd::k_eq_project_tc, qfd::kEtSmem);
+}
 #endif
 
 // The transform passes of one codeword (2^logm message entries in 2^(logm -
@@ -1119,8 +1123,25 @@ static void device_point_table(cudaStream_t s, const std::vector<F>& point, W we
 static std::vector<F> eq_slice(const std::vector<F>& p) { return equality_table(p); }
 static std::vector<F> tensor_slice(const std::vector<F>& p) { return tensor_weights(p); }
 
+// Whether the equality projection of nb blocks of m elements runs on tcgen05
+// (kernels/eq_mma.cuh).  Its time hardly depends on nb (the MMA takes eight
+// blocks' rows either way), the CUDA-core kernels' does.  Measured on B200, us,
+// tcgen05 / CUDA cores, F65521 then KoalaBear:
+//   8 blocks   2^12  9 / 18, 9 / 24      2^20  33 / 49, 33 / 76
+//              2^27  1769 / 4435, 2864 / 6269
+//   4 blocks   2^14  10 / 13, 12 / 15    2^20  28 / 30, 32 / 42
+//              2^22  55 / 87, 68 / 117
+//   4 blocks   2^16  17 / 13, 19 / 18    2^18  21 / 13, 23 / 17: a few stages
+//              per CTA, one after the other, against four CTAs per SM
+//   1 block    2^20  22 / 15, 26 / 20
+// Bulk copies take 16-byte aligned weights.
+static bool eq_on_tcgen05(uint64_t m, int nb, uint64_t block_bytes, const void* weights) {
+  if (nb < 4 || m % (2 * qfd::kEtPairs) || (m > (1u << 14) && m < (1u << 20))) return false;
+  return block_bytes % 16 == 0 && reinterpret_cast<uintptr_t>(weights) % 16 == 0;
+}
+
 // Raw lane sums of blocks [b0, b0 + nb) (nb <= 8) against the equality table
-// in weights_: the tensor-core kernel for F65521, else the IMAD one.
+// in weights_.
 void GpuBackend::eq_project_launch(const W* bva, uint64_t active, uint64_t b0, int nb, unsigned long long* raw,
                                    unsigned grid) {
   constexpr int L = F::kLanes;
@@ -1134,6 +1155,13 @@ void GpuBackend::eq_project_launch(const W* bva, uint64_t active, uint64_t b0, i
     return;
   }
 #endif
+  if (eq_on_tcgen05(m, nb, P_.block_len * sizeof(W), bva)) {
+    const uint32_t stages = uint32_t(m / (2 * qfd::kEtPairs));
+    QF_LAUNCH(s_, "k_eq_project_tc", bytes,
+              qfd::k_eq_project_tc<<<tile_grid(stages), qfd::kEtThreads, qfd::kEtSmem, s_>>>(
+                  bva, active, P_.block_len, b0, nb, stages, weights_.p, raw, transform_error()));
+    return;
+  }
 #if defined(QF_FIELD_KB)
   QF_LAUNCH(s_, "k_eq_project_blocks", bytes,
             qfd::k_eq_project_blocks<<<grid, qfd::kEqThreads, 0, s_>>>(bva, active, P_.block_len, b0, nb, m, weights_.p, raw));
@@ -1169,6 +1197,7 @@ std::vector<std::vector<F>> GpuBackend::project_blocks(const std::vector<F>& out
   std::vector<unsigned long long> h(kRaw * nblocks);
   QF_CK(cudaMemcpyAsync(h.data(), raw.p, h.size() * 8, cudaMemcpyDeviceToHost, s_));
   QF_CK(cudaStreamSynchronize(s_));
+  check_transforms();
   // Entries are two's complement sums of exact signed totals below 2^63.
   std::vector<std::vector<F>> out(nblocks, std::vector<F>(L));
   for (size_t b = 0; b < nblocks; ++b)
