@@ -14,6 +14,7 @@
 #include "intops.h"
 
 #include <algorithm>
+#include <list>
 #include <map>
 #include <mutex>
 #include <set>
@@ -2029,16 +2030,29 @@ F GpuBackend::eo_build(const Query<F>& q, F ch, F inv, size_t logical, size_t st
   } else {
     eo_witness_launch(bva_, active_, rows, stride, dp.p, wit_.p);
   }
-  // Query fold (tbv.rs:393-428): zero, then two disjoint passes of large-term
-  // tiles, then the merged small-term contributions.
+  // Query fold (tbv.rs:393-428): zero, then passes of large-term tiles, then
+  // the merged small-term contributions.  k_query_terms adds without atomics,
+  // so the terms of a pass are disjoint.  Claim and zero-suffix terms are, in
+  // the first pass; a padding term overlaps the claim's, and the column
+  // rectangles of one matrix's padding overlap each other (each spans its rows'
+  // whole width, with zero factors inside): each goes to the first pass that
+  // holds nothing in its rows.
   QF_CK(cudaMemsetAsync(qv_.p, 0, rows * 16, s_));
   std::vector<F> powers = consecutive_powers(ch, stride);
   const size_t ls = ilog2(stride);
   TableBuilder tb;
-  std::vector<qfd::TermTiles> pass_terms[2];
-  uint64_t pass_tiles[2] = {0, 0}, query_bytes[2] = {0, 0};
+  struct Pass {
+    std::vector<qfd::TermTiles> terms;
+    std::map<uint64_t, uint64_t> spans;  // first row -> end
+    uint64_t tiles = 0, bytes = 0;
+    DBuf<qfd::TermTiles> dev;
+    bool holds(uint64_t first, uint64_t end) const {
+      auto it = spans.lower_bound(end);
+      return it != spans.begin() && std::prev(it)->second > first;
+    }
+  };
+  std::list<Pass> passes(1);
   std::map<uint64_t, F> sparse;
-  const size_t n_claim_terms = P_.layout.buckets.size();
   for (size_t ti = 0; ti < q.terms.size(); ++ti) {
     const Term<F>& term = q.terms[ti];
     if (term.len() >= stride) {
@@ -2047,15 +2061,17 @@ F GpuBackend::eo_build(const Query<F>& q, F ch, F inv, size_t logical, size_t st
       for (size_t j = 0; j < stride; ++j) sc += low[j] * powers[j];
       sc = term.scale * sc;
       if (sc.is_zero()) continue;
-      // Claim and zero-suffix terms are disjoint; padding terms overlap claim terms.
-      const int pass = (ti < n_claim_terms || term.offset >= P_.layout.active) ? 0 : 1;
+      const uint64_t first = term.offset / stride, n = term.len() / stride;
+      auto pass = passes.begin();
+      while (pass->holds(first, first + n))
+        if (++pass == passes.end()) pass = passes.emplace(passes.end());
+      pass->spans[first] = first + n;
       const size_t nh = term.factors.size() - ls;
-      qfd::TermTiles T = term_tiles(tb, term.factors.data() + ls, nh, term.offset / stride, term.len() / stride,
-                                    uint32_t(pass_tiles[pass]), sc);
-      pass_tiles[pass] += term_tile_count(T);
-      check(pass_tiles[pass] < (uint64_t(1) << 31), "query tile count");
-      query_bytes[pass] += T.rows * 32;
-      pass_terms[pass].push_back(T);
+      qfd::TermTiles T = term_tiles(tb, term.factors.data() + ls, nh, first, n, uint32_t(pass->tiles), sc);
+      pass->tiles += term_tile_count(T);
+      check(pass->tiles < (uint64_t(1) << 31), "query tile count");
+      pass->bytes += T.rows * 32;
+      pass->terms.push_back(T);
     } else {
       for (size_t i = 0; i < term.len(); ++i) {
         auto it = sparse.find(term.offset / stride);
@@ -2066,27 +2082,26 @@ F GpuBackend::eo_build(const Query<F>& q, F ch, F inv, size_t logical, size_t st
   }
   DBuf<Fe> tables;
   tb.build(s_, tables);
-  DBuf<qfd::TermTiles> dtt[2];
-  for (int pass = 0; pass < 2; ++pass) {
-    auto& tl = pass_terms[pass];
+  for (Pass& pass : passes) {
+    auto& tl = pass.terms;
     if (tl.empty()) continue;
-    dtt[pass].alloc(tl.size());
+    pass.dev.alloc(tl.size());
     if (KernelOptions::per_matrix) {  // one launch per term, tiles renumbered from 0
       std::vector<qfd::TermTiles> solo = tl;
       for (auto& T : solo) T.first_tile = 0;
-      QF_CK(cudaMemcpyAsync(dtt[pass].p, solo.data(), solo.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
+      QF_CK(cudaMemcpyAsync(pass.dev.p, solo.data(), solo.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
       for (size_t k = 0; k < tl.size(); ++k) {
         const uint64_t n = term_tile_count(tl[k]);
         QF_LAUNCH(s_, "k_query_terms", tl[k].rows * 32,
                   qfd::k_query_terms<<<unsigned((n + qfd::kTilesPerCta - 1) / qfd::kTilesPerCta), kThreads, 0, s_>>>(
-                      dtt[pass].p + k, 1, uint32_t(n), tables.p, qv_.p));
+                      pass.dev.p + k, 1, uint32_t(n), tables.p, qv_.p));
       }
       continue;
     }
-    QF_CK(cudaMemcpyAsync(dtt[pass].p, tl.data(), tl.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
-    QF_LAUNCH(s_, "k_query_terms", query_bytes[pass],
-              qfd::k_query_terms<<<unsigned((pass_tiles[pass] + qfd::kTilesPerCta - 1) / qfd::kTilesPerCta), kThreads, 0, s_>>>(
-                  dtt[pass].p, int(tl.size()), uint32_t(pass_tiles[pass]), tables.p, qv_.p));
+    QF_CK(cudaMemcpyAsync(pass.dev.p, tl.data(), tl.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
+    QF_LAUNCH(s_, "k_query_terms", pass.bytes,
+              qfd::k_query_terms<<<unsigned((pass.tiles + qfd::kTilesPerCta - 1) / qfd::kTilesPerCta), kThreads, 0, s_>>>(
+                  pass.dev.p, int(tl.size()), uint32_t(pass.tiles), tables.p, qv_.p));
   }
   if (!sparse.empty()) {
     std::vector<uint64_t> idx;
