@@ -727,7 +727,7 @@ def main():
                 "peak_source": "pinned 2 GiB host->device copy, best of 3, measured in this run"}
 
     # The exact integer-limb tensor-core forms of the weight passes against
-    # the dp4a / IMAD kernels the library runs (F65521): one more profiled
+    # the kernels the library runs (F65521: dp4a, tcgen05): one more profiled
     # step with them switched on, same bytes.
     imma_cmp = None
     if not sixteen and not args.no_compare:
@@ -741,7 +741,7 @@ def main():
         assert pr_on.to_bytes() == proof.to_bytes(), "tensor-core path proof bytes differ"
         off = stats
         pairs = {"eo_witness": ("k_eo_witness_mma", "k_eo_witness"), "block_fold": ("k_block_fold_mma", "k_block_fold"),
-                 "eq_projection": ("k_eq_project_mma", "k_eq_project_blocks")}
+                 "eq_projection": ("k_eq_project_mma", "k_eq_project_tc")}
         imma_cmp = {}
         for name, (on_k, off_k) in pairs.items():
             a, b = on_stats.get(on_k), off.get(off_k)
@@ -750,7 +750,7 @@ def main():
                                   "imma_hbm_frac": a["bytes"] / (a["ms"] / 1000.0) / 1e9 / peak,
                                   "dp4a_hbm_frac": b["bytes"] / (b["ms"] / 1000.0) / 1e9 / peak}
         imma_cmp["what"] = ("per-step kernel time of the exact integer-limb tensor-core kernels (mma.sync s8 x u8 -> "
-                            "s32) against the dp4a / IMAD kernels, same proof bytes")
+                            "s32) against the library's kernels (dp4a; the eq projection tcgen05), same proof bytes")
 
     # The extension-product sums of the EO, sumcheck and LiteBullet rounds on
     # the tensor cores against the CUDA-core kernels: two more profiled steps,
