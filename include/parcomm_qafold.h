@@ -83,7 +83,8 @@ void qf_committed_free(qf_committed* committed);
  * (for weight sets larger than HBM; page-locked memory lets the copies
  * overlap the compute) or in device memory (weights resident, codewords
  * recomputed: a pool of many commitments; its producer must have finished
- * writing it, as for qf_commit).  It stays owned by the caller and must stay
+ * writing it, as for qf_commit; at an 8-byte boundary, else QF_E_ARGUMENT, and
+ * at a 16-byte one for qf_range_audit).  It stays owned by the caller and must stay
  * valid and unchanged until the committed handle is freed.  Every pass that reads the
  * weights (commit, EO cross terms and witness, projection, block fold) stages
  * them into HBM one PCS block at a time, and binding re-encodes each block
@@ -222,8 +223,8 @@ size_t qf_last_error(char* buf, size_t cap);
  * Writes the root of PCS block `block` (the bytes qf_commit writes at
  * roots_out + 32 * block) to the 32 device bytes `d_root`, asynchronously on
  * `stream` (a cudaStream_t; NULL is the legacy default stream).  `d_bva` is
- * a device pointer to the n_values active int8 entries.  Unlike qf_commit it
- * neither copies the weights nor checks the layout's zero padding.
+ * a device pointer to the n_values active int8 entries, at an 8-byte boundary
+ * (QF_E_ARGUMENT otherwise).  Unlike qf_commit it neither copies the weights nor checks the layout's zero padding.
  *
  * Limit: F65521 blocks of at most 2^QF_NOALLOC_MAX_CHUNK_LOG weights
  * (config chunk_log <= 20); larger blocks return QF_E_ARGUMENT.  All working

@@ -349,7 +349,7 @@ class Parameters:
         every pass; `resident_bytes` of leading blocks are kept in HBM after
         the first pass (None: as many as the device's free memory allows next
         to the proof's own peak).  A CUDA tensor stays where it is and is read
-        in place.  The weights must stay unchanged while the handle lives.
+        in place; it must start at an 8-byte boundary.  The weights must stay unchanged while the handle lives.
         The roots, claims and proof bytes equal those of `commit`."""
         if hasattr(values, "data_ptr"):
             if int(values.element_size()) != np.dtype(self.weight_dtype).itemsize or not values.is_contiguous():

@@ -22,21 +22,23 @@ const Parameters<F>& params_of(const qf_params* p) { return *static_cast<const P
 
 // Any zero-padding entry that is nonzero sets the flag (Layout::validate_values,
 // layout.rs:136-155).  Segments are at most kZeroPiece bytes; a CTA checks one
-// with 16-byte loads over its aligned middle and byte loads at the ends.
+// with 16-byte loads over its middle, aligned by address, and byte loads at the ends.
 constexpr uint64_t kZeroPiece = 4096;
 __global__ void k_check_zero_segments(const uint8_t* __restrict__ bva, const uint64_t* __restrict__ seg, uint32_t n_seg,
                                       unsigned int* __restrict__ flag) {
   bool bad = false;
   for (uint32_t s = blockIdx.x; s < n_seg; s += gridDim.x) {
-    const uint64_t a = seg[2 * s], b = seg[2 * s + 1];
-    const uint64_t a16 = (a + 15) & ~uint64_t(15), b16 = b & ~uint64_t(15);
+    const uint8_t* const a = bva + seg[2 * s];
+    const uint8_t* const b = bva + seg[2 * s + 1];
+    const uint8_t* const a16 = a + (-reinterpret_cast<uintptr_t>(a) & 15);
+    const uint8_t* const b16 = b - (reinterpret_cast<uintptr_t>(b) & 15);
     if (a16 >= b16) {
-      for (uint64_t i = a + threadIdx.x; i < b; i += blockDim.x) bad |= bva[i] != 0;
+      for (const uint8_t* p = a + threadIdx.x; p < b; p += blockDim.x) bad |= *p != 0;
     } else {
-      for (uint64_t i = a + threadIdx.x; i < a16; i += blockDim.x) bad |= bva[i] != 0;
-      for (uint64_t i = b16 + threadIdx.x; i < b; i += blockDim.x) bad |= bva[i] != 0;
-      for (uint64_t i = a16 + 16 * uint64_t(threadIdx.x); i < b16; i += 16 * uint64_t(blockDim.x)) {
-        const uint4 u = *reinterpret_cast<const uint4*>(bva + i);
+      for (const uint8_t* p = a + threadIdx.x; p < a16; p += blockDim.x) bad |= *p != 0;
+      for (const uint8_t* p = b16 + threadIdx.x; p < b; p += blockDim.x) bad |= *p != 0;
+      for (const uint8_t* p = a16 + 16 * threadIdx.x; p < b16; p += 16 * blockDim.x) {
+        const uint4 u = *reinterpret_cast<const uint4*>(p);
         bad |= (u.x | u.y | u.z | u.w) != 0;
       }
     }
@@ -284,6 +286,7 @@ void commit_streamed(const qf_params* params, const void* host, uint64_t n_value
   auto t0 = std::chrono::steady_clock::now();
   const size_t resident = size_t(resident_budget(P, resident_bytes) / (P.block_len * sizeof(W)));
   c->src = std::make_unique<BlockStream>(static_cast<const W*>(host), n_values, P.block_len, resident, 3);
+  if (c->src->on_device()) check_weight_alignment(static_cast<const W*>(host), n_values);
   c->be = std::make_unique<GpuBackend>(P, c->src.get(), c->stream, static_cast<DeviceTables*>(params->tables.get()));
   // Padding segments of every live block, relative to the block, uploaded once.
   const size_t live = c->src->live_blocks();

@@ -1009,6 +1009,12 @@ std::vector<Digest> GpuBackend::commit_streamed(const BlockStream::BlockFn& per_
   return roots_;
 }
 
+void check_weight_alignment(const W* d_bva, uint64_t active) {
+  const uintptr_t need = active >= 8 / sizeof(W) ? 8 : (active >= 4 ? 4 : 1);
+  if (reinterpret_cast<uintptr_t>(d_bva) % need)
+    fail(QF_E_ARGUMENT, "device weights must lie at a " + std::to_string(need) + "-byte boundary");
+}
+
 // The same kernels as commit_block + encode_and_hash, launched without the
 // per-launch timers and into caller-owned buffers.
 void commit_block_into(const Parameters<F>& P, const W* d_bva, uint64_t active, size_t b, Fe* cw, uint4* tree,

@@ -104,6 +104,11 @@ class BlockStream {
   uint64_t copied_ = 0;
 };
 
+// Refuses device weights that are read in place and not at an 8-byte boundary,
+// the widest unit that the kernels load without a look at the address (four
+// bytes where there are fewer than eight).
+void check_weight_alignment(const W* d_bva, uint64_t active);
+
 // Commitment root of block `b` of a device BVA (`active` entries), computed
 // only in the caller's device buffers: `cw` holds 2R x cols entries, `tree`
 // 4 x 2R words (2 x 2R digests), `alpha` the R entries of the top code's

@@ -260,7 +260,8 @@ __global__ void __launch_bounds__(kTermThreads) k_project_terms16(const int8_t* 
 // ---------------------------------------------------------------- EO
 // witness[row] = sum_lane v[row * stride + lane] * inv^lane (eo.rs:119-132).
 // Packed EO witness (eo.rs:119-132): witness[row] = sum_lane v(row * stride +
-// lane) * inv_powers[lane].  For stride 16 a row is one 16-byte load and each
+// lane) * inv_powers[lane].  For stride 16 a row is one 16-byte load (two of 8
+// bytes where the weights lie at an 8-byte boundary only) and each
 // coefficient two chains of four dp4a (signed weights against the low and
 // high bytes of the powers, held in registers); |sum| < 16 * 128 * 65520.
 __global__ void k_eo_witness(const int8_t* __restrict__ bva, uint64_t active, uint64_t rows, int stride,
@@ -278,15 +279,22 @@ __global__ void k_eo_witness(const int8_t* __restrict__ bva, uint64_t active, ui
   // kWitRows rows per thread and iteration, their loads issued first, so that
   // enough 16-byte loads are in flight to keep HBM busy.
   constexpr int kWitRows = 4;
+  const bool aligned = reinterpret_cast<uintptr_t>(bva) % 16 == 0;
   const uint64_t nthr = uint64_t(gridDim.x) * blockDim.x;
   for (uint64_t row0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; row0 < rows; row0 += kWitRows * nthr) {
     uint4 raw[kWitRows];
 #pragma unroll
     for (int q = 0; q < kWitRows; ++q) {
       const uint64_t row = row0 + q * nthr;
-      raw[q] = (stride == 16 && row < rows && row * 16 + 16 <= active)
-                   ? *reinterpret_cast<const uint4*>(bva + row * 16)
-                   : make_uint4(0, 0, 0, 0);
+      raw[q] = make_uint4(0, 0, 0, 0);
+      if (stride == 16 && row < rows && row * 16 + 16 <= active) {
+        if (aligned) {
+          raw[q] = *reinterpret_cast<const uint4*>(bva + row * 16);
+        } else {
+          const uint2 a = *reinterpret_cast<const uint2*>(bva + row * 16), b = *reinterpret_cast<const uint2*>(bva + row * 16 + 8);
+          raw[q] = make_uint4(a.x, a.y, b.x, b.y);
+        }
+      }
     }
 #pragma unroll
     for (int q = 0; q < kWitRows; ++q) {
@@ -341,10 +349,18 @@ __global__ void k_eo_witness(const int8_t* __restrict__ bva, uint64_t active, ui
 constexpr size_t kEqWeightSmem = 2 * (kEqChunk / 2) * 16;  // the weight double buffer of k_eq_project_blocks
 
 // 16 bytes of weights from global to shared memory, asynchronously; bytes at
-// or past `avail` (0..16) are zero-filled (and not read).
-__device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, uint32_t avail) {
+// or past `avail` (0..16) are zero-filled (and not read).  Not `aligned`: in
+// two halves, from an 8-byte boundary.
+__device__ __forceinline__ void cp_async16_zfill(void* smem, const int8_t* gmem, uint32_t avail, bool aligned) {
   const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem), "r"(avail) : "memory");
+  if (aligned) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem), "r"(avail) : "memory");
+  } else {
+    const uint32_t first = avail < 8 ? avail : 8;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sa), "l"(gmem), "r"(first) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sa + 8), "l"(avail > 8 ? gmem + 8 : gmem), "r"(avail - first)
+                 : "memory");
+  }
 }
 
 __global__ void __launch_bounds__(kEqThreads, 2) k_eq_project_blocks(const int8_t* __restrict__ bva, uint64_t active,
@@ -363,6 +379,7 @@ __global__ void __launch_bounds__(kEqThreads, 2) k_eq_project_blocks(const int8_
   __shared__ long long tot_s[kEqBlocks][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = threadIdx.x & 1;
   for (int t = threadIdx.x; t < kEqBlocks * 64; t += kEqThreads) tot_s[t >> 6][t & 63] = 0;
+  const bool aligned = reinterpret_cast<uintptr_t>(bva) % 16 == 0;
   // Issues the copies of block b's chunk into wts_s[buf].
   auto stage_block = [&](uint64_t c0, int b, int buf) {
     const uint64_t bbase = (first_block + b) * block_len;
@@ -372,7 +389,7 @@ __global__ void __launch_bounds__(kEqThreads, 2) k_eq_project_blocks(const int8_
       uint32_t avail = 0;
       if (i < m && g < active) avail = uint32_t(active - g < 16 ? active - g : 16);
       if (i + 1 >= m && avail > 8) avail = 8;  // the second element is past the packed length
-      cp_async16_zfill(&wts_s[buf][u], avail ? static_cast<const void*>(bva + g) : static_cast<const void*>(bva), avail);
+      cp_async16_zfill(&wts_s[buf][u], avail ? bva + g : bva, avail, aligned);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };

@@ -152,21 +152,23 @@ __device__ __forceinline__ void witness_row(const Wt* __restrict__ row, const Fe
 
 // Packed EO witness (eo.rs:119-132): witness[row] = sum_lane v(row * stride +
 // lane) * inv_powers[lane], stride <= 64, so a sum is below 2^52.  Full rows
-// of 16 or 64 payloads take the unrolled path; the rest the generic loop.
+// of 16 or 64 payloads take the unrolled path (weights at a 16-byte boundary);
+// the rest the generic loop, which loads 8 bytes.
 __global__ void __launch_bounds__(256, 2) k_eo_witness(const Wt* __restrict__ bva, uint64_t active, uint64_t rows,
                                                        int stride, const Fe* __restrict__ inv_powers,
                                                        Fe* __restrict__ witness) {
   __shared__ Fe pw[64];
   if (threadIdx.x < stride) pw[threadIdx.x] = inv_powers[threadIdx.x];
   __syncthreads();
+  const bool aligned = reinterpret_cast<uintptr_t>(bva) % 16 == 0;
   for (uint64_t row = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; row < rows; row += uint64_t(gridDim.x) * blockDim.x) {
     long long acc[kC];
 #pragma unroll
     for (int k = 0; k < kC; ++k) acc[k] = 0;
     const uint64_t g0 = row * stride;
-    if (stride == 16 && g0 + 16 <= active) {
+    if (aligned && stride == 16 && g0 + 16 <= active) {
       witness_row<16>(bva + g0, pw, acc);
-    } else if (stride == 64 && g0 + 64 <= active) {
+    } else if (aligned && stride == 64 && g0 + 64 <= active) {
       witness_row<64>(bva + g0, pw, acc);
     } else if (g0 < active) {
       for (int l0 = 0; l0 < stride; l0 += 4) {

@@ -123,6 +123,7 @@ extern "C" int qf_commit_block_noalloc(const qf_params* params, const int8_t* d_
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     if ((n_values && !on_device(d_bva, dev)) || !on_device(d_root, dev))
       fail(QF_E_ARGUMENT, "qf_commit_block_noalloc: d_bva and d_root must be memory of the current device");
+    qfg::check_weight_alignment(d_bva, n_values);
     int sdev = dev;
     if (cudaStreamGetDevice(s, &sdev) == cudaSuccess && sdev != dev)
       fail(QF_E_ARGUMENT, "qf_commit_block_noalloc: the stream belongs to another device");
