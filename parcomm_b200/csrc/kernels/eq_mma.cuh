@@ -201,6 +201,10 @@ __global__ void __launch_bounds__(kEtThreads, 1) k_eq_project_tc(const Wt* __res
       tc5::mma_commit(unused(s));
       if (n % kEtGroup == kEtGroup - 1 || n + 1 == n_own) tc5::mma_commit(full(g & 1));
     }
+    // No MMA is in flight and no arrival on its way when the CTA ends, also
+    // after a wait that gave up.
+    for (uint32_t i = n_own < kEtStages ? 0 : n_own - kEtStages; i < n_own; ++i) tc5::mbar_wait(unused(i % kEtStages), i / kEtStages & 1);
+    for (uint32_t g = n_groups < 2 ? 0 : n_groups - 2; g < n_groups; ++g) tc5::mbar_wait(full(g & 1), g >> 1 & 1);
   }
   __syncwarp();
   tc5::fence_before_sync();

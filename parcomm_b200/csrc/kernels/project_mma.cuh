@@ -165,6 +165,11 @@ __global__ void __launch_bounds__(kPmThreads, 1) k_project_terms_mma(const int8_
       }
       tc5::mma_commit(full(k & 1));
     }
+    // No MMA is in flight and no arrival on its way when the CTA ends, also
+    // after a wait that gave up.
+    const uint32_t k1 = g1 - g0;
+    for (uint32_t i = n < kPmStages ? 0 : n - kPmStages; i < n; ++i) tc5::mbar_wait(unused(i % kPmStages), i / kPmStages & 1);
+    for (uint32_t k = k1 < 2 ? 0 : k1 - 2; k < k1; ++k) tc5::mbar_wait(full(k & 1), k >> 1 & 1);
   }
   __syncwarp();
   tc5::fence_before_sync();

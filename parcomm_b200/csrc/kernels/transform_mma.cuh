@@ -376,8 +376,8 @@ __global__ void __launch_bounds__(tc_threads(SRC), 1) k_transform(const __grid_c
               const uint32_t b = x ? reg[c] * kTcRegionBytes + (uint32_t(j) << 13) : reg[j] * kTcRegionBytes + (uint32_t(c) << 13);
               tc5::mma_i8(tmem0 + 256u * (c & 1), desc_a + ((a + 32u * j) >> 4), desc_b + (b >> 4), tc5::idesc_i8(128, 256), j > 0);
             }
-            tc5::mma_commit(B.full(c & 1));
             if (last) tc5::mma_commit(B.unused(reg[c]));
+            tc5::mma_commit(B.full(c & 1));
           }
           if (!last) ++w;
         }
@@ -385,6 +385,16 @@ __global__ void __launch_bounds__(tc_threads(SRC), 1) k_transform(const __grid_c
 #pragma unroll
         for (int j = 0; j < 4; ++j) lap[j] += reg[j] + 4 >= NR ? 1 : 0;
         r0 = tc_next<NR>(r0);
+      }
+      // No MMA is in flight and no arrival on its way when the CTA ends, also
+      // after a wait that gave up (the last tile's regions are four back).
+      if (u > 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t r = r0 + j + NR - 4, reg = r >= NR ? r - NR : r;
+          tc5::mbar_wait(B.unused(reg), (lap[j] - (reg + 4 >= NR ? 1 : 0)) & 1);
+        }
+        for (uint32_t i = u - 2; i < u; ++i) tc5::mbar_wait(B.full(i & 1), i >> 1 & 1);
       }
     }
     __syncwarp();
