@@ -162,9 +162,8 @@ std::vector<F> DeviceCodeword::entries() const {
   return h;
 }
 
-// The tensor-core transform passes (F65521), below.
-static void configure_transforms();
-static void check_transforms();
+// The tensor-core kernels' shared memory, below.
+static void configure_tcgen05();
 
 // Planar tile kernels take up to 2^kMaxTileLog elements (128 KiB of shared
 // memory); the opt-in is set once per device.
@@ -188,7 +187,7 @@ static void configure_tile_kernels() {
   // 38 KiB of static shared memory plus the 32 KiB weight double buffer.
   set_smem(qfd::k_eq_project_blocks, qfd::kEqWeightSmem);
 #endif
-  configure_transforms();
+  configure_tcgen05();
   done.insert(dev);
 }
 
@@ -526,21 +525,6 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
   }
 }
 
-// A wait that gave up in a tensor-core kernel: one flag per process in host memory
-// that the device can write.
-static int* transform_error() {
-  static int* flag = [] {
-    int* p = nullptr;
-    QF_CK(cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
-    *p = 0;
-    return p;
-  }();
-  return flag;
-}
-static void check_transforms() {
-  if (*static_cast<volatile int*>(transform_error())) fail(QF_E_CUDA, "CUDA: a tensor-core kernel gave up waiting");
-}
-
 #if !defined(QF_FIELD_KB)
 // ---------------------------------------------------------------- tensor-core transform passes
 // Codewords of at least 2^23 message entries run their tile passes and the
@@ -564,8 +548,9 @@ template <int CFG, int SRC, int OP1, int OP2, int MID, bool HASY>
 struct Transform {
   static constexpr int kMats = (HASY ? 2 : 1) * (OP2 >= 0 && OP1 != OP2 ? 2 : 1);
   static void configure() { set_smem(qfd::k_transform<CFG, SRC, OP1, OP2, MID, HASY>, qfd::tc_smem(kMats)); }
-  static void run(cudaStream_t s, qfd::TcPass& p) {
-    p.error = transform_error();
+  static void run(cudaStream_t s, qfd::TcPass& p, WaitFlag* waits) {
+    check(waits != nullptr, "tensor-core passes need an owner of their waits");
+    p.error = waits->word();
     qfd::k_transform<CFG, SRC, OP1, OP2, MID, HASY><<<tile_grid(p.n_tiles), qfd::tc_threads(SRC), qfd::tc_smem(kMats), s>>>(p);
   }
 };
@@ -576,8 +561,7 @@ using StridedWht = Transform<qfd::kStridedCfg, qfd::kTcElements, qfd::kWht, -1, 
 using MobiusWht = Transform<qfd::kStridedCfg, qfd::kTcElements, qfd::kMobius, qfd::kWht, qfd::kMidStore, true>;
 using MobiusWhtShort = Transform<qfd::kStridedCfg, qfd::kTcElements, qfd::kMobius, qfd::kWht, qfd::kMidStore, false>;
 
-static void configure_transforms() {
-  transform_error();
+static void configure_tcgen05() {
   PackMobius::configure();
   CopyMobius::configure();
   WhtAlphaWht::configure();
@@ -641,8 +625,7 @@ static qfd::TcPass strided_pass(const void* src, Fe* dst, int logR, int logm, in
   return p;
 }
 #else
-static void configure_transforms() {
-  transform_error();
+static void configure_tcgen05() {
   set_smem(qfd::k_eq_project_tc, qfd::kEtSmem);
 }
 #endif
@@ -670,8 +653,11 @@ static void configure_transforms() {
 // pass's register stages; its Mobius levels then join pass 1 and its WHT
 // levels run as a strided pass from the message into the parity.  Columns
 // shorter than one tile (logR < 12) take one tile pass per WHT.
+//
+// `waits` belongs to the caller, who checks it after the passes; null where the
+// codeword is too small for the tensor-core passes.
 static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int logm, int mob_from, bool timed,
-                          bool allow_tuning) {
+                          bool allow_tuning, WaitFlag* waits) {
   check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
   const size_t R = size_t(1) << logR;
   Fe* msg = cw;
@@ -707,7 +693,7 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
         } else {
           qfd::TcPass p = strided_pass(src, par, logR, logm, from, levels);
           launch(s, timed, "k_transform_wht", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0),
-                 [&] { StridedWht::run(s, p); });
+                 [&] { StridedWht::run(s, p, waits); });
         }
         src = par;
         from += levels;
@@ -719,8 +705,8 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
         qfd::TcPass p = strided_pass(msg, par, logR, logm, kT, k);
         p.mid = msg;
         launch(s, timed, "k_transform_mobius_wht", 3 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, k > 5 ? 4 : 2, 0), [&] {
-          if (k > 5) MobiusWht::run(s, p);
-          else MobiusWhtShort::run(s, p);
+          if (k > 5) MobiusWht::run(s, p, waits);
+          else MobiusWhtShort::run(s, p, waits);
         });
       }
       wht(par, top);
@@ -731,7 +717,7 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
     p.alpha = alpha;
     p.col_log = logm - logR;
     launch(s, timed, "k_transform_wht_alpha_wht", 2 * n * 16 + uint64_t(R) * 16, qf_intops::transform_ops(kOps, n, 0, 0, 4, 1),
-           [&] { WhtAlphaWht::run(s, p); });
+           [&] { WhtAlphaWht::run(s, p, waits); });
     wht(par, kT);
     return;
   }
@@ -785,7 +771,8 @@ static int first_mobius_levels(int logm, int logR) {
 }
 // Packed weights of one block (from entry src_base of the `active` at bva)
 // with their first Mobius levels into the message half at cw.
-static void pack_mobius(cudaStream_t s, bool timed, const W* bva, uint64_t active, uint64_t src_base, Fe* cw, int logR, int logm) {
+static void pack_mobius(cudaStream_t s, bool timed, const W* bva, uint64_t active, uint64_t src_base, Fe* cw, int logR, int logm,
+                        WaitFlag* waits) {
   check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
   const int l0 = first_mobius_levels(logm, logR);
   const uint64_t n = uint64_t(1) << logm, bytes = n * (F::kLanes * sizeof(W) + 16);
@@ -794,7 +781,7 @@ static void pack_mobius(cudaStream_t s, bool timed, const W* bva, uint64_t activ
     qfd::TcPass p = tile_pass(bva, cw, logR, logm);
     p.active = active;
     p.src_base = src_base;
-    launch(s, timed, "k_transform_pack_mobius", bytes, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0), [&] { PackMobius::run(s, p); });
+    launch(s, timed, "k_transform_pack_mobius", bytes, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0), [&] { PackMobius::run(s, p, waits); });
     return;
   }
 #endif
@@ -804,14 +791,14 @@ static void pack_mobius(cudaStream_t s, bool timed, const W* bva, uint64_t activ
   });
 }
 // The same from an element vector (the block-folded table).
-static void copy_mobius(cudaStream_t s, const Fe* src, Fe* cw, int logR, int logm) {
+static void copy_mobius(cudaStream_t s, const Fe* src, Fe* cw, int logR, int logm, WaitFlag* waits) {
   check(logm <= 30, "transform passes index a codeword of at most 2^31 elements");
   const int l0 = first_mobius_levels(logm, logR);
   const uint64_t n = uint64_t(1) << logm;
 #if !defined(QF_FIELD_KB)
   if (mma_transforms(logm, logR)) {
     qfd::TcPass p = tile_pass(src, cw, logR, logm);
-    launch(s, true, "k_transform_copy_mobius", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0), [&] { CopyMobius::run(s, p); });
+    launch(s, true, "k_transform_copy_mobius", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0), [&] { CopyMobius::run(s, p, waits); });
     return;
   }
 #endif
@@ -865,7 +852,7 @@ static void build_tree(cudaStream_t s, uint4* tree, uint64_t n_leaves, std::vect
 // Encode (see encode_passes), then leaf hashes and tree.
 void GpuBackend::encode_and_hash(DeviceCodeword& out, const Fe* alpha, int logR, int logm, bool ext_domain, int mob_from) {
   const size_t R = size_t(1) << logR;
-  encode_passes(s_, out.cw.p, alpha, logR, logm, mob_from < 0 ? logm : mob_from, true, true);
+  encode_passes(s_, out.cw.p, alpha, logR, logm, mob_from < 0 ? logm : mob_from, true, true, &waits_);
   // Leaves and inner levels.
   const uint64_t n_ext = 2 * R;
   ::qfd::LeafPrefix lp = leaf_prefix(out.n_cols, ext_domain);
@@ -881,7 +868,7 @@ void GpuBackend::encode_and_hash(DeviceCodeword& out, const Fe* alpha, int logR,
   uint4 r[2];
   QF_CK(cudaMemcpyAsync(r, out.tree.p + 2 * out.level_off.back(), 32, cudaMemcpyDeviceToHost, s_));
   QF_CK(cudaStreamSynchronize(s_));
-  check_transforms();
+  waits_.check();
   out.root_ = digest_from_words(r);
 }
 
@@ -918,6 +905,7 @@ bool DeviceSetup::encode_level(const QaCode<F>& target, const QaCode<F>& current
   cudaStream_t s;
   QF_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   {
+    WaitFlag waits(wait_words());
     DBuf<Fe> cw(er * hc), alpha(mr);
     DBuf<uint4> lv(2 * er);
     // Column col is the message current.alphas[col / rf][(col % rf) mr ..][.. mr).
@@ -926,7 +914,7 @@ bool DeviceSetup::encode_level(const QaCode<F>& target, const QaCode<F>& current
                             cudaMemcpyHostToDevice, s));
     QF_CK(cudaMemcpyAsync(alpha.p, target.alphas[1].data(), mr * 16, cudaMemcpyHostToDevice, s));
     const int logm = ilog2(mr * hc);
-    encode_passes(s, cw.p, alpha.p, ilog2(mr), logm, logm, false, true);
+    encode_passes(s, cw.p, alpha.p, ilog2(mr), logm, logm, false, true, &waits);
     const ::qfd::SetupLeafPrefix pf = setup_leaf_prefix(shape);
     qfd::k_hash_setup_rows<<<unsigned((er + kThreads - 1) / kThreads), kThreads, 0, s>>>(cw.p, er, int(hc), pf, lv.p);
     QF_CK(cudaGetLastError());
@@ -935,7 +923,7 @@ bool DeviceSetup::encode_level(const QaCode<F>& target, const QaCode<F>& current
     QF_CK(cudaMemcpyAsync(encoded.data(), cw.p, er * hc * 16, cudaMemcpyDeviceToHost, s));
     QF_CK(cudaMemcpyAsync(leaves.data(), lv.p, er * 32, cudaMemcpyDeviceToHost, s));
     QF_CK(cudaStreamSynchronize(s));
-    check_transforms();
+    waits.check();
   }
   QF_CK(cudaStreamDestroy(s));
   return true;
@@ -954,7 +942,7 @@ static std::unique_ptr<DeviceCodeword> alloc_codeword(size_t R, size_t cols, cud
 Digest GpuBackend::encode_block(const W* bva, uint64_t active, uint64_t src_base, DeviceCodeword& cw) {
   const int logm = ilog2(P_.pcs.packed_len());
   const int logR = logm - ilog2(P_.pcs.pp->extension_columns);
-  pack_mobius(s_, true, bva, active, src_base, cw.cw.p, logR, logm);
+  pack_mobius(s_, true, bva, active, src_base, cw.cw.p, logR, logm, &waits_);
   encode_and_hash(cw, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, first_mobius_levels(logm, logR));
   return cw.root_;
 }
@@ -1026,8 +1014,8 @@ void commit_block_into(const Parameters<F>& P, const W* d_bva, uint64_t active, 
   const size_t R = size_t(1) << logR;
   check(P.pcs.pp->seq.top().message_len == R, "alpha table length");
   // Message half: pack + the first Mobius levels, then the rest of the encode.
-  pack_mobius(s, false, d_bva, active, uint64_t(b) * P.block_len, cw, logR, logm);
-  encode_passes(s, cw, alpha, logR, logm, first_mobius_levels(logm, logR), false, false);
+  pack_mobius(s, false, d_bva, active, uint64_t(b) * P.block_len, cw, logR, logm, nullptr);
+  encode_passes(s, cw, alpha, logR, logm, first_mobius_levels(logm, logR), false, false, nullptr);
   // Row leaves, inner levels, root.
   const uint64_t n_ext = 2 * R;
   const unsigned lthreads = qfd::leaf_threads(n_ext);
@@ -1166,7 +1154,7 @@ void GpuBackend::eq_project_launch(const W* bva, uint64_t active, uint64_t b0, i
     const uint32_t stages = uint32_t(m / (2 * qfd::kEtPairs));
     QF_LAUNCH(s_, "k_eq_project_tc", bytes,
               qfd::k_eq_project_tc<<<tile_grid(stages), qfd::kEtThreads, qfd::kEtSmem, s_>>>(
-                  bva, active, P_.block_len, b0, nb, stages, weights_.p, raw, transform_error()));
+                  bva, active, P_.block_len, b0, nb, stages, weights_.p, raw, waits_.word()));
     return;
   }
 #if defined(QF_FIELD_KB)
@@ -1204,7 +1192,7 @@ std::vector<std::vector<F>> GpuBackend::project_blocks(const std::vector<F>& out
   std::vector<unsigned long long> h(kRaw * nblocks);
   QF_CK(cudaMemcpyAsync(h.data(), raw.p, h.size() * 8, cudaMemcpyDeviceToHost, s_));
   QF_CK(cudaStreamSynchronize(s_));
-  check_transforms();
+  waits_.check();
   // Entries are two's complement sums of exact signed totals below 2^63.
   std::vector<std::vector<F>> out(nblocks, std::vector<F>(L));
   for (size_t b = 0; b < nblocks; ++b)
@@ -1317,7 +1305,7 @@ Digest GpuBackend::fold_and_commit(const std::vector<F>& fw) {
     block_fold_launch(bva_, active_, blocks, dT.p, 0);
   }
   folded_ = alloc_codeword(size_t(1) << logR, P_.pcs.pp->extension_columns, s_);
-  copy_mobius(s_, values_.p, folded_->cw.p, logR, logm);
+  copy_mobius(s_, values_.p, folded_->cw.p, logR, logm, &waits_);
   encode_and_hash(*folded_, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, first_mobius_levels(logm, logR));
   host_v_.clear();
   host_w_.clear();
@@ -1570,7 +1558,7 @@ Digest GpuBackend::commit_folded_values(const std::vector<F>& values) {
   values_.alloc(m);
   QF_CK(cudaMemcpyAsync(values_.p, values.data(), m * 16, cudaMemcpyHostToDevice, s_));
   folded_ = alloc_codeword(size_t(1) << logR, P_.pcs.pp->extension_columns, s_);
-  copy_mobius(s_, values_.p, folded_->cw.p, logR, logm);
+  copy_mobius(s_, values_.p, folded_->cw.p, logR, logm, &waits_);
   encode_and_hash(*folded_, tables_->top_alpha1(*P_.pcs.pp), logR, logm, false, first_mobius_levels(logm, logR));
   QF_CK(cudaStreamSynchronize(s_));  // the host copy of `values` may go once this returns
   host_v_.clear();
@@ -1834,7 +1822,7 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
     std::vector<F> h(np * lanes_of[g]);
     QF_CK(cudaMemcpyAsync(h.data(), dpiece.p, h.size() * 16, cudaMemcpyDeviceToHost, s_));
     QF_CK(cudaStreamSynchronize(s_));
-    check_transforms();
+    waits_.check();
     for (size_t k = 0; k < np; ++k)
       for (size_t l = 0; l < lanes_of[g]; ++l) out[g][seg_term[g][k]][l] += h[k * lanes_of[g] + l];
   }
@@ -1852,7 +1840,7 @@ void GpuBackend::project_terms_launch(const W* bva, uint64_t active, const qfd::
   if (groups && reinterpret_cast<uintptr_t>(bva) % 16 == 0) {
     QF_LAUNCH(s_, "k_project_terms", bytes,
               qfd::k_project_terms_mma<<<tile_grid(groups), qfd::kPmThreads, qfd::kPmSmem, s_>>>(bva, terms, n_terms, groups, tables, out,
-                                                                                           transform_error()));
+                                                                                           waits_.word()));
     return;
   }
   if (lanes == 16) {
@@ -1927,7 +1915,7 @@ std::vector<std::vector<F>> GpuBackend::project_terms(const std::vector<const Te
   std::vector<F> h(terms.size() * common_lanes);
   QF_CK(cudaMemcpyAsync(h.data(), dterm.p, h.size() * 16, cudaMemcpyDeviceToHost, s_));
   QF_CK(cudaStreamSynchronize(s_));
-  check_transforms();
+  waits_.check();
   for (size_t t = 0; t < terms.size(); ++t)
     for (size_t l = 0; l < common_lanes; ++l) out[t][l] = h[t * common_lanes + l];
   return out;

@@ -269,6 +269,7 @@ class GpuBackend : public Backend<F>,
   void eo_witness_launch(const W* bva, uint64_t active, uint64_t rows, size_t stride, const Fe* powers, Fe* out);
 
   const Parameters<F>& P_;
+  WaitFlag waits_{wait_words()};  // of this backend's tensor-core launches
   const W* bva_;              // resident weights, or null
   BlockStream* src_ = nullptr;  // streamed weights, or null
   std::unique_ptr<DeviceCodeword> scratch_;  // re-encoded block of a streamed backend

@@ -113,6 +113,22 @@ PinnedStage::Lease PinnedStage::acquire(size_t bytes) {
   return l;
 }
 
+WaitWords& wait_words() {
+  static WaitWords words(
+      [] {
+        void* p = nullptr;
+        QF_CK(cudaHostAlloc(&p, WaitWords::kPage * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+        return static_cast<int*>(p);
+      },
+      [](const int* page) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, page) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        return false;
+      });
+  return words;
+}
+
 size_t DevicePool::cached_bytes() {
   const int dev = current_device();
   std::lock_guard<std::mutex> g(g_pool_mu);

@@ -17,6 +17,7 @@
 #include "device/hash_prefix.h"
 #include "host/protocol.h"
 #include "host/sections.h"
+#include "host/wait_flag.h"
 
 namespace qfg {
 using namespace qf;
@@ -115,6 +116,10 @@ struct PinnedStage {
   };
   static Lease acquire(size_t bytes);
 };
+
+// Words for the waits of tensor-core kernels (host/wait_flag.h), in page-locked
+// memory that every device writes.
+WaitWords& wait_words();
 
 template <class T>
 struct DBuf {
