@@ -95,6 +95,11 @@ __global__ void __launch_bounds__(kPmThreads, 1) k_project_terms_mma(const int8_
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tail + 8 * (2 * kPmStages + 4));
   const uint32_t g0 = uint32_t(uint64_t(n_groups) * blockIdx.x / gridDim.x), g1 = uint32_t(uint64_t(n_groups) * (blockIdx.x + 1) / gridDim.x);
   int ti = 0;
+  for (int last = n_terms - 1; ti < last;) {  // the entry of group g0
+    const int mid = (ti + last + 1) >> 1;
+    if (terms[mid].first_group <= g0) ti = mid;
+    else last = mid - 1;
+  }
 
   if (warp < kPmEpiWarps) {
     // Thread m: lane m & 15 of the group's tile m >> 4.
