@@ -1691,25 +1691,59 @@ qfd::TermTiles term_tiles(TableBuilder& tb, const std::array<F, 2>* f, size_t nh
 uint64_t term_tile_count(const qfd::TermTiles& T) { return (T.rows + (uint64_t(1) << T.lb) - 1) >> T.lb; }
 
 // Numbers the groups of a launch's list (its `n` entries hold `tiles` tiles,
-// over `active` weights) for the tensor-core projection; 0 when the list is
+// over `active` weights) for the tensor-core projection; none when the list is
 // not for it: lanes other than 16, or an entry that reaches past the weights
 // or starts off a row of 16 (its rows are copied 16 bytes at a time).
-uint32_t plan_groups(qfd::TermTiles* t, size_t n, uint64_t tiles, uint64_t active, size_t lanes) {
-  uint32_t groups = 0;
+qfd::TermGroups plan_groups(qfd::TermTiles* t, size_t n, uint64_t tiles, uint64_t active, size_t lanes) {
+  qfd::TermGroups G;
   for (size_t k = 0; k < n; ++k) t[k].tiles = uint32_t((k + 1 < n ? t[k + 1].first_tile : tiles) - t[k].first_tile);
 #if !defined(QF_FIELD_KB)
-  if (lanes != 16) return 0;
+  if (lanes != 16) return G;
+  // A stage takes about as long with one tile as with eight, and a group about
+  // two stages more: runs of equal cost per CTA.  Runs of equal length left
+  // lists of terms of many sizes, largest first, to the first CTAs: 40 matrices
+  // of 500 x 1000, proof, took 100 us instead of 48 (dp4a kernel 55).
+  struct Run {
+    uint32_t first, n;
+    uint64_t cost;  // of each
+  };
+  std::vector<Run> runs;
+  uint64_t total = 0;
+  uint32_t groups = 0;
+  auto run = [&](uint32_t count, uint64_t rows) {
+    if (!count) return;
+    runs.push_back({groups, count, 2 + qfd::pm_stages(rows)});
+    groups += count;
+    total += count * runs.back().cost;
+  };
   for (size_t k = 0; k < n; ++k) {
     const uint64_t rows = std::min<uint64_t>(t[k].rows, (uint64_t(t[k].tile_skip) + t[k].tiles) << t[k].lb);
-    if (t[k].offset % 16 || t[k].offset + rows * 16 > active) return 0;
+    if (t[k].offset % 16 || t[k].offset + rows * 16 > active) return G;
     t[k].first_group = groups;
-    groups += qfd::pm_groups(t[k]);
+    const bool ragged = qfd::pm_ragged(t[k]);
+    run(qfd::pm_groups(t[k]) - (ragged ? 1 : 0), uint64_t(1) << t[k].lb);
+    run(ragged ? 1 : 0, t[k].rows & ((uint64_t(1) << t[k].lb) - 1));
   }
+  G.n = groups;
+  G.ctas = std::min(tile_grid(groups), qfd::kPmCtas);
+  uint64_t before = 0;  // cost of the runs passed
+  uint32_t c = 0;
+  for (const Run& r : runs) {
+    // CTA c starts at the group whose middle is the first at or past its share.
+    for (; c < G.ctas; ++c) {
+      const uint64_t share = total * c / G.ctas, at = share > before ? share - before : 0;
+      const uint64_t skip = (at + r.cost / 2) / r.cost;
+      if (skip >= r.n) break;
+      G.first[c] = r.first + uint32_t(skip);
+    }
+    before += r.n * r.cost;
+  }
+  for (; c <= G.ctas; ++c) G.first[c] = groups;
 #else
   (void)active;
   (void)lanes;
 #endif
-  return groups;
+  return G;
 }
 }  // namespace
 
@@ -1779,7 +1813,7 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
   // outputs block-major too, so a piece's tiles are one segment.
   std::vector<qfd::TermTiles> all;
   std::vector<std::vector<size_t>> piece_at(live, std::vector<size_t>(G));
-  std::vector<std::vector<uint32_t>> groups_bg(live, std::vector<uint32_t>(G, 0));
+  std::vector<std::vector<qfd::TermGroups>> groups_bg(live, std::vector<qfd::TermGroups>(G));
   std::vector<std::vector<uint64_t>> tile_base(live, std::vector<uint64_t>(G));
   std::vector<uint64_t> tiles_g(G, 0);
   std::vector<std::vector<uint32_t>> seg(G, std::vector<uint32_t>(1, 0));
@@ -1834,13 +1868,13 @@ std::vector<std::vector<std::vector<F>>> GpuBackend::project_groups_streamed(
 // (plan_groups) and the weights are 16-byte aligned (HBM-bound), else the dp4a
 // kernel; other lane widths and KoalaBear: the general one.
 void GpuBackend::project_terms_launch(const W* bva, uint64_t active, const qfd::TermTiles* terms, int n_terms,
-                                      uint64_t tiles, uint32_t groups, const Fe* tables, size_t lanes, Fe* out, uint64_t bytes) {
+                                      uint64_t tiles, const qfd::TermGroups& groups, const Fe* tables, size_t lanes, Fe* out, uint64_t bytes) {
   const unsigned grid = unsigned((tiles + qfd::kTilesPerCta - 1) / qfd::kTilesPerCta);
 #if !defined(QF_FIELD_KB)
-  if (groups && reinterpret_cast<uintptr_t>(bva) % 16 == 0) {
+  if (groups.n && reinterpret_cast<uintptr_t>(bva) % 16 == 0) {
     QF_LAUNCH(s_, "k_project_terms", bytes,
-              qfd::k_project_terms_mma<<<tile_grid(groups), qfd::kPmThreads, qfd::kPmSmem, s_>>>(bva, terms, n_terms, groups, tables, out,
-                                                                                           waits_.word()));
+              qfd::k_project_terms_mma<<<groups.ctas, qfd::kPmThreads, qfd::kPmSmem, s_>>>(bva, terms, n_terms, groups, tables, out,
+                                                                                        waits_.word()));
     return;
   }
   if (lanes == 16) {
@@ -1895,7 +1929,7 @@ std::vector<std::vector<F>> GpuBackend::project_terms(const std::vector<const Te
     // One launch per term (a bucket's claim term, or a padding / suffix
     // term): each term's tiles renumbered from 0, its outputs at its first tile.
     std::vector<qfd::TermTiles> solo = tt;
-    std::vector<uint32_t> groups;
+    std::vector<qfd::TermGroups> groups;
     for (auto& T : solo) {
       T.first_tile = 0;
       groups.push_back(plan_groups(&T, 1, term_tile_count(T), active_, common_lanes));
@@ -1907,7 +1941,7 @@ std::vector<std::vector<F>> GpuBackend::project_terms(const std::vector<const Te
                            dtile.p + size_t(tt[k].first_tile) * common_lanes, tt[k].rows * common_lanes * sizeof(W) + n * 16);
     }
   } else {
-    const uint32_t groups = plan_groups(tt.data(), tt.size(), tiles, active_, common_lanes);
+    const qfd::TermGroups groups = plan_groups(tt.data(), tt.size(), tiles, active_, common_lanes);
     QF_CK(cudaMemcpyAsync(dtt.p, tt.data(), tt.size() * sizeof(qfd::TermTiles), cudaMemcpyHostToDevice, s_));
     project_terms_launch(bva_, active_, dtt.p, int(tt.size()), tiles, groups, tables.p, common_lanes, dtile.p, proj_bytes);
   }

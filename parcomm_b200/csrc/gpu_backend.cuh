@@ -11,7 +11,8 @@
 #include "gpu_common.cuh"
 
 namespace QFD_NS {
-struct TermTiles;  // kernels/open.cuh
+struct TermTiles;   // kernels/open.cuh
+struct TermGroups;  // kernels/open.cuh
 }
 
 namespace QFB_NS {
@@ -264,7 +265,7 @@ class GpuBackend : public Backend<F>,
   std::vector<F> copy_to_host(const Fe* p, uint64_t n);
   void block_fold_launch(const W* bva, uint64_t active, int blocks, const Fe* T, int accumulate);
   void project_terms_launch(const W* bva, uint64_t active, const qfd::TermTiles* terms, int n_terms, uint64_t tiles,
-                            uint32_t groups, const Fe* tables, size_t lanes, Fe* out, uint64_t bytes);
+                            const qfd::TermGroups& groups, const Fe* tables, size_t lanes, Fe* out, uint64_t bytes);
   void eq_project_launch(const W* bva, uint64_t active, uint64_t b0, int nb, unsigned long long* raw, unsigned grid);
   void eo_witness_launch(const W* bva, uint64_t active, uint64_t rows, size_t stride, const Fe* powers, Fe* out);
 

@@ -120,6 +120,13 @@ struct TermTiles {
   uint32_t lb, mb;
   uint32_t tiles, first_group;  // tiles of this list entry, and its first group of eight (tensor-core projection)
 };
+// The groups of a launch of the tensor-core projection: none, or their number
+// and the first group of each CTA (of `ctas`).
+constexpr uint32_t kPmCtas = 192;
+struct TermGroups {
+  uint32_t n = 0, ctas = 0;
+  uint32_t first[kPmCtas + 1];
+};
 __device__ __forceinline__ int find_term(const TermTiles* __restrict__ t, int n, uint32_t tile) {
   int lo = 0, hi = n - 1;
   while (lo < hi) {

@@ -37,6 +37,8 @@ __host__ __device__ inline uint32_t pm_groups(const TermTiles& T) {
   const uint32_t full = T.tiles - (pm_ragged(T) ? 1 : 0);
   return (full + kPmTiles - 1) / kPmTiles + (pm_ragged(T) ? 1 : 0);
 }
+// Stages of a group of tiles of `rows` rows.
+__host__ __device__ inline uint32_t pm_stages(uint64_t rows) { return uint32_t((rows + kPmRows - 1) / kPmRows); }
 struct PmGroup {
   TermTiles T;
   uint32_t first, tiles;  // tiles of the entry
@@ -53,11 +55,10 @@ __device__ __forceinline__ PmGroup pm_group(const TermTiles* __restrict__ terms,
   return G;
 }
 
-// The groups over the grid, a run of them per CTA.  Every row of every entry
-// lies below the end of the weights, and the weights and offsets are 16-byte
+// A run of the groups per CTA (list.first).  Every row of every entry lies below the end of the weights, and the weights and offsets are 16-byte
 // aligned (the launcher checks both).
 __global__ void __launch_bounds__(kPmThreads, 1) k_project_terms_mma(const int8_t* __restrict__ bva, const TermTiles* __restrict__ terms,
-                                                                     int n_terms, uint32_t n_groups,
+                                                                     int n_terms, const __grid_constant__ TermGroups list,
                                                                      const Fe* __restrict__ tables, Fe* __restrict__ out, int* error) {
   extern __shared__ unsigned char pm_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(pm_raw) + 1023) & ~uintptr_t(1023));
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(kPmThreads, 1) k_project_terms_mma(const int8_
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tail + 8 * (2 * kPmStages + 4));
-  const uint32_t g0 = uint32_t(uint64_t(n_groups) * blockIdx.x / gridDim.x), g1 = uint32_t(uint64_t(n_groups) * (blockIdx.x + 1) / gridDim.x);
+  const uint32_t g0 = list.first[blockIdx.x], g1 = list.first[blockIdx.x + 1];
   int ti = 0;
   for (int last = n_terms - 1; ti < last;) {  // the entry of group g0
     const int mid = (ti + last + 1) >> 1;

@@ -18,6 +18,7 @@ pytestmark = pytest.mark.gpu
     ([(64, 64)] * 300 + [(37, 50)] * 40, 17),
     ([(500, 1000)] * 3 + [(90, 72)] * 60 + [(5, 3)] * 20, 18),
     ([(1100, 1024)] + [(16, 48)] * 150, 17),
+    ([(16, 16)] * 3 + [(5000, 1024)], 20),
 ])
 def test_lists_of_many_terms(shapes, chunk_log):
     rng = np.random.default_rng(len(shapes))
