@@ -386,8 +386,14 @@ static void wht_tile_launch(cudaStream_t s, const Fe* src, Fe* dst, const Fe* al
 
 // Codewords of fewer than 2^19 message entries have fewer 4096-element tiles
 // than the chip has SMs, and a pass takes as long as one tile: their tiles
-// shrink to 1/128 of the message, 64 elements at least.
-static int small_tile_log(int logm) { return std::max(6, std::min(qfd::kMaxTileLog, logm - 7)); }
+// shrink to 1/128 of the message.  Up to 2^12 entries one tile takes the whole
+// Mobius transform in one launch, and a second launch costs more than the
+// smaller tiles save (root of one F65521 block, us, one tile / 64-element tiles
+// and a second pass: 2^7 36.4 / 40.5, 2^10 45.1 / 47.4, 2^12 52.0 / 52.2; at 2^13
+// two passes are needed either way, 67.7 / 59.4).
+static int small_tile_log(int logm) {
+  return logm <= qfd::kMaxTileLog ? logm : std::min(qfd::kMaxTileLog, std::max(6, logm - 7));
+}
 
 // 2^cb consecutive group bases per tile of a k-level strided pass: 64-byte
 // runs at k = 10, the full 4096-element tile below that (small messages: as
