@@ -185,7 +185,8 @@ static void configure_tile_kernels() {
   set_smem(qfd::k_wht_alpha_wht_tile, bytes + qfd::kAlphaStageSmem);
 #if !defined(QF_FIELD_KB)
   // 38 KiB of static shared memory plus the 32 KiB weight double buffer.
-  set_smem(qfd::k_eq_project_blocks, qfd::kEqWeightSmem);
+  set_smem(qfd::k_eq_project_blocks<true>, qfd::kEqWeightSmem);
+  set_smem(qfd::k_eq_project_blocks<false>, qfd::kEqWeightSmem);
 #endif
   configure_tcgen05();
   done.insert(dev);
@@ -1167,9 +1168,9 @@ void GpuBackend::eq_project_launch(const W* bva, uint64_t active, uint64_t b0, i
   QF_LAUNCH(s_, "k_eq_project_blocks", bytes,
             qfd::k_eq_project_blocks<<<grid, qfd::kEqThreads, 0, s_>>>(bva, active, P_.block_len, b0, nb, m, weights_.p, raw));
 #else
+  const auto kernel = reinterpret_cast<uintptr_t>(bva) % 16 ? qfd::k_eq_project_blocks<false> : qfd::k_eq_project_blocks<true>;
   QF_LAUNCH(s_, "k_eq_project_blocks", bytes,
-            qfd::k_eq_project_blocks<<<grid, qfd::kEqThreads, qfd::kEqWeightSmem, s_>>>(bva, active, P_.block_len, b0, nb, m,
-                                                                                     weights_.p, raw));
+            kernel<<<grid, qfd::kEqThreads, qfd::kEqWeightSmem, s_>>>(bva, active, P_.block_len, b0, nb, m, weights_.p, raw));
 #endif
 }
 

@@ -349,11 +349,12 @@ __global__ void k_eo_witness(const int8_t* __restrict__ bva, uint64_t active, ui
 constexpr size_t kEqWeightSmem = 2 * (kEqChunk / 2) * 16;  // the weight double buffer of k_eq_project_blocks
 
 // 16 bytes of weights from global to shared memory, asynchronously; bytes at
-// or past `avail` (0..16) are zero-filled (and not read).  Not `aligned`: in
+// or past `avail` (0..16) are zero-filled (and not read).  Not ALIGNED: in
 // two halves, from an 8-byte boundary.
-__device__ __forceinline__ void cp_async16_zfill(void* smem, const int8_t* gmem, uint32_t avail, bool aligned) {
+template <bool ALIGNED>
+__device__ __forceinline__ void cp_async16_zfill(void* smem, const int8_t* gmem, uint32_t avail) {
   const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  if (aligned) {
+  if (ALIGNED) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem), "r"(avail) : "memory");
   } else {
     const uint32_t first = avail < 8 ? avail : 8;
@@ -363,6 +364,9 @@ __device__ __forceinline__ void cp_async16_zfill(void* smem, const int8_t* gmem,
   }
 }
 
+// ALIGNED: the weights lie at a 16-byte boundary (the choice inside the copy
+// loop made the kernel 6 % slower).
+template <bool ALIGNED>
 __global__ void __launch_bounds__(kEqThreads, 2) k_eq_project_blocks(const int8_t* __restrict__ bva, uint64_t active,
                                                                     uint64_t block_len, uint64_t first_block, int nb,
                                                                     uint64_t m, const Fe* __restrict__ weights,
@@ -379,7 +383,6 @@ __global__ void __launch_bounds__(kEqThreads, 2) k_eq_project_blocks(const int8_
   __shared__ long long tot_s[kEqBlocks][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = threadIdx.x & 1;
   for (int t = threadIdx.x; t < kEqBlocks * 64; t += kEqThreads) tot_s[t >> 6][t & 63] = 0;
-  const bool aligned = reinterpret_cast<uintptr_t>(bva) % 16 == 0;
   // Issues the copies of block b's chunk into wts_s[buf].
   auto stage_block = [&](uint64_t c0, int b, int buf) {
     const uint64_t bbase = (first_block + b) * block_len;
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(kEqThreads, 2) k_eq_project_blocks(const int8_
       uint32_t avail = 0;
       if (i < m && g < active) avail = uint32_t(active - g < 16 ? active - g : 16);
       if (i + 1 >= m && avail > 8) avail = 8;  // the second element is past the packed length
-      cp_async16_zfill(&wts_s[buf][u], avail ? bva + g : bva, avail, aligned);
+      cp_async16_zfill<ALIGNED>(&wts_s[buf][u], avail ? bva + g : bva, avail);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
