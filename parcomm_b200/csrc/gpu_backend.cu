@@ -181,7 +181,6 @@ static void configure_tile_kernels() {
   set_smem(qfd::k_wht_tile<true>, bytes);
   set_smem(qfd::k_butterfly_strided<qfd::kMobius>, bytes);
   set_smem(qfd::k_butterfly_strided<qfd::kWht>, bytes);
-  set_smem(qfd::k_mobius_wht_strided, bytes + qfd::kPrefetchSmem);
   set_smem(qfd::k_wht_alpha_wht_tile, bytes + qfd::kAlphaStageSmem);
 #if !defined(QF_FIELD_KB)
   // 38 KiB of static shared memory plus the 32 KiB weight double buffer.
@@ -549,7 +548,10 @@ static void strided_passes(cudaStream_t s, const Fe* src, Fe* dst, int logR, int
 // A KoalaBear pass costs the same time here, but its butterflies work on half
 // as many coefficients (0.26, 0.45, 0.59 at 2^25): it keeps them.
 static constexpr int kMmaMinLogm = 23;
-static bool mma_transforms(int logm, int logR) { return logm >= kMmaMinLogm && logR >= qfd::kTcTileLog; }
+// Rows of 2^13 to 2^22: a tile's levels and at most nine strided ones.
+static bool mma_transforms(int logm, int logR) {
+  return logm >= kMmaMinLogm && logR >= qfd::kTcTileLog && logR < qfd::kTcTileLog + 10;
+}
 
 template <int CFG, int SRC, int OP1, int OP2, int MID, bool HASY>
 struct Transform {
@@ -601,10 +603,10 @@ static qfd::TcPass tile_pass(const void* src, Fe* dst, int logR, int logm) {
 // contraction) is a run too.  A single stage (k <= 5) is X, its levels in its
 // upper slots.
 static qfd::TcPass strided_pass(const void* src, Fe* dst, int logR, int logm, int lo, int k) {
-  static constexpr int kRuns[13] = {0, 1, 2, 12, 3, 7, 8, 4, 9, 5, 10, 6, 11}, kRuns3[3] = {0, 1, 12};
+  static constexpr int kRuns[7] = {0, 1, 2, 12, 3, 7, 8};
   static constexpr int kContractY[7] = {0, 1, 7, 8, 9, 10, 11};
   const int runs = qfd::kTcTileLog - k;
-  check(k >= 1 && k <= 10 && lo >= runs, "strided transform pass");
+  check(k >= 1 && k <= 9 && lo >= runs, "strided transform pass");
   qfd::TcPass p{};
   p.src = src;
   p.dst = dst;
@@ -620,7 +622,7 @@ static qfd::TcPass strided_pass(const void* src, Fe* dst, int logR, int logm, in
     p.stride[slot] = index_stride(bit, logR);
   };
   for (int j = 0; j < runs; ++j)
-    place(k <= 5 ? (j < 7 - k ? j : j + k) : (runs == 3 ? kRuns3[j] : kRuns[j]), j);
+    place(k <= 5 ? (j < 7 - k ? j : j + k) : kRuns[j], j);
   for (int j = 0, slot = 0; j < k; ++j) {
     while (used[slot]) ++slot;
     place(slot, lo + j);
@@ -647,19 +649,18 @@ static void configure_tcgen05() {
 // 975-1002).
 //
 // Every level is a 2 x 2 map on one index bit, and maps on different bits
-// commute, so the passes group them by the bits a tile covers (12 per tile;
-// the tile levels 0..11 of a column are its low 12 bits):
-//   1. Mobius on the bits above the fused span (the column bits [logR, logm),
-//      plus any within-column bits above 22), strided, in place;
-//   2. Mobius then WHT #1 on the fused span [12, min(logR, 22)) in one
-//      strided pass, writing the message (now final) and the parity;
-//   3. WHT #1 on within-column bits above 22 (KoalaBear, logR = 23);
-//   4. WHT #1 on bits 0..11, alpha, WHT #2 on bits 0..11: one tile pass;
-//   5. WHT #2 on [12, logR), strided.
-// A fused span of fewer than 6 levels leaves too few bits for the fused
-// pass's register stages; its Mobius levels then join pass 1 and its WHT
-// levels run as a strided pass from the message into the parity.  Columns
-// shorter than one tile (logR < 12) take one tile pass per WHT.
+// commute, so the passes group them by the bits a tile covers (the tile levels
+// of a column are its low 12 bits, 13 on the tensor cores):
+//   1. Mobius on the bits that the first pass left, strided, in place;
+//   2. WHT #1 on [12, logR), strided, from the message into the parity;
+//   3. WHT #1 on bits 0..11, alpha, WHT #2 on bits 0..11: one tile pass;
+//   4. WHT #2 on [12, logR), strided.
+// On the tensor cores (mma_transforms) pass 1 takes the column bits [logR,
+// logm) only, and pass 2 the Mobius levels [13, logR) with the WHT's, storing
+// the message too.  The butterflies keep them apart: a pass of both is bound by
+// issue where two strided ones run at 0.95 of HBM (KoalaBear, 8B step: 351
+// against 337 ms).  Columns shorter than one tile (logR < 12) take one tile pass
+// per WHT.
 //
 // `waits` belongs to the caller, who checks it after the passes; null where the
 // codeword is too small for the tensor-core passes.
@@ -686,80 +687,51 @@ static void encode_passes(cudaStream_t s, Fe* cw, const Fe* alpha, int logR, int
   }
 #if !defined(QF_FIELD_KB)
   if (mma_transforms(logm, logR)) {
-    // The same passes over tiles of 13 bits on the tensor cores; spans of five
-    // levels or fewer are bound by HBM and stay with the butterflies.
+    // The same passes over tiles of 13 bits on the tensor cores.  Block
+    // codewords have 32 columns, so k is 5..9; the setup's levels need no Mobius
+    // transform.  Five WHT levels or fewer on their own are bound by HBM and
+    // stay with the butterflies.
     constexpr int kT = qfd::kTcTileLog;
-    check(!mobius || mob_from == kT, "the Mobius tile pass covers bits 0..12");
+    const int k = logR - kT;
+    check(!mobius || (mob_from == kT && k >= 5), "tensor-core Mobius passes: rows");
     const uint64_t n = uint64_t(1) << logm;
-    const int top = std::min(logR, kT + 10), k = top - kT;
-    auto wht = [&](const Fe* src, int from) {  // levels [from, logR) into the parity
-      while (from < logR) {
-        const int span = logR - from, levels = span > 10 ? span / 2 : span;
-        if (levels <= 5) {
-          strided_passes<qfd::kWht>(s, src, par, logR, logm, from, from + levels, timed, allow_tuning);
-        } else {
-          qfd::TcPass p = strided_pass(src, par, logR, logm, from, levels);
-          launch(s, timed, "k_transform_wht", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0),
-                 [&] { StridedWht::run(s, p, waits); });
-        }
-        src = par;
-        from += levels;
+    auto wht = [&](const Fe* src) {  // levels [13, logR) into the parity
+      if (k <= 5) {
+        strided_passes<qfd::kWht>(s, src, par, logR, logm, kT, logR, timed, allow_tuning);
+      } else {
+        qfd::TcPass p = strided_pass(src, par, logR, logm, kT, k);
+        launch(s, timed, "k_transform_wht", 2 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, 2, 0),
+               [&] { StridedWht::run(s, p, waits); });
       }
     };
     if (mobius) {
-      strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, top, logm, timed, allow_tuning);
-      if (k > 0) {
-        qfd::TcPass p = strided_pass(msg, par, logR, logm, kT, k);
-        p.mid = msg;
-        launch(s, timed, "k_transform_mobius_wht", 3 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, k > 5 ? 4 : 2, 0), [&] {
-          if (k > 5) MobiusWht::run(s, p, waits);
-          else MobiusWhtShort::run(s, p, waits);
-        });
-      }
-      wht(par, top);
+      strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, logR, logm, timed, allow_tuning);
+      qfd::TcPass p = strided_pass(msg, par, logR, logm, kT, k);
+      p.mid = msg;
+      launch(s, timed, "k_transform_mobius_wht", 3 * n * 16, qf_intops::transform_ops(kOps, n, 0, 0, k > 5 ? 4 : 2, 0), [&] {
+        if (k > 5) MobiusWht::run(s, p, waits);
+        else MobiusWhtShort::run(s, p, waits);
+      });
     } else {
-      wht(msg, kT);
+      wht(msg);
     }
     qfd::TcPass p = tile_pass(k > 0 ? par : msg, par, logR, logm);
     p.alpha = alpha;
     p.col_log = logm - logR;
     launch(s, timed, "k_transform_wht_alpha_wht", 2 * n * 16 + uint64_t(R) * 16, qf_intops::transform_ops(kOps, n, 0, 0, 4, 1),
            [&] { WhtAlphaWht::run(s, p, waits); });
-    wht(par, kT);
+    wht(par);
     return;
   }
 #endif
   constexpr int kT = qfd::kMaxTileLog;
-  const int top = std::min(logR, kT + 10);  // fused span [kT, top)
-  const int k = top - kT;
-  // KoalaBear does not fuse the Mobius and WHT #1 strided levels: its
-  // butterflies reduce at every level (3 operations per element, coefficient
-  // and level), so a 20-level pass is issue-bound where its separate strided
-  // passes run at 0.95 of HBM (the fused plan measured 351 against 337 ms
-  // per 8B step).  It still takes the WHT-alpha-WHT tile pass.
-#if defined(QF_FIELD_KB)
-  const bool fused = false;
-#else
-  const bool fused = mobius && k >= 6;
-#endif
-  check(!fused || mob_from == kT, "the Mobius tile pass covers bits 0..11");
-  if (mobius) strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, fused ? top : mob_from, logm, timed, allow_tuning);
-  if (fused) {
-    const int cb = strided_cb(k, logm);
-    const uint32_t tiles = uint32_t(uint64_t(1) << (logm - k - cb));
-    launch(s, timed, "k_mobius_wht_strided", (uint64_t(3) << logm) * 16,
-           qf_intops::transform_ops(kOps, uint64_t(1) << logm, k, k, 2, 0), [&] {
-             qfd::k_mobius_wht_strided<<<tile_grid(tiles), qfd::kTileThreads, qfd::kTileSmem + qfd::kPrefetchSmem, s>>>(cw, uint32_t(R), logR,
-                                                                                                 kT, k, cb, tiles);
-           });
-    strided_passes<qfd::kWht>(s, par, par, logR, logm, top, logR, timed, allow_tuning);
-  } else {
-    // WHT #1's levels [12, logR) as one span (the tuner's split), message
-    // into parity.
-    strided_passes<qfd::kWht>(s, msg, par, logR, logm, kT, logR, timed, allow_tuning);
-  }
+  // The Mobius transform's other levels in place, then WHT #1's levels
+  // [12, logR) from the message into the parity, each as one span (the tuner's
+  // split).
+  if (mobius) strided_passes<qfd::kMobius>(s, msg, msg, logR, logm, mob_from, logm, timed, allow_tuning);
+  strided_passes<qfd::kWht>(s, msg, par, logR, logm, kT, logR, timed, allow_tuning);
   const uint32_t tiles = uint32_t(uint64_t(1) << (logm - kT));
-  const Fe* src = k > 0 ? par : msg;
+  const Fe* src = logR > kT ? par : msg;
   launch(s, timed, "k_wht_alpha_wht_tile", (uint64_t(2) << logm) * 16 + uint64_t(R) * 16,
          qf_intops::transform_ops(kOps, uint64_t(1) << logm, 2 * kT, 0, 2, 1), [&] {
            qfd::k_wht_alpha_wht_tile<<<tile_grid(tiles), qfd::kTileThreads, qfd::kTileSmem + qfd::kAlphaStageSmem, s>>>(

@@ -380,37 +380,6 @@ __device__ __forceinline__ void window_stage_r(uint4* t, int b, int r, int lvl) 
   else window_stage<OP, 1>(t, b, lvl);
 }
 
-// The last window of a pass: OP's levels, reduction to canonical form,
-// fin(e, Fr&) on each element (a store to HBM, or the step between two
-// transforms), and (PUT) the result back into the tile.
-template <int OP, int R, bool PUT, class Fin>
-__device__ __forceinline__ void window_last(uint4* t, int b, int lvl, Fin fin) {
-  int off[1 << R];
-  window_offsets<R>(b, off);
-  for (int g = threadIdx.x; g < (kTile >> R); g += blockDim.x) {
-    const int base = group_base(g, b, R);
-    uint32_t v[1 << R][kC];
-    group_get<R>(t, base, off, v);
-    reg_levels<OP, R>(v, lvl);
-#pragma unroll
-    for (int j = 0; j < (1 << R); ++j) {
-      Fr w;
-#pragma unroll
-      for (int c = 0; c < kC; ++c) w.c[c] = tile_final(v[j][c]);
-      fin(base + (j << b), w);
-#pragma unroll
-      for (int c = 0; c < kC; ++c) v[j][c] = w.c[c];
-    }
-    if (PUT) group_put<R>(t, base, off, v);
-  }
-}
-template <int OP, bool PUT, class Fin>
-__device__ __forceinline__ void window_last_r(uint4* t, int b, int r, int lvl, Fin fin) {
-  if (r == 3) window_last<OP, 3, PUT>(t, b, lvl, fin);
-  else if (r == 2) window_last<OP, 2, PUT>(t, b, lvl, fin);
-  else window_last<OP, 1, PUT>(t, b, lvl, fin);
-}
-
 // The window where a fused pass changes transforms: OP1's levels, reduction,
 // step(e, Fr&) on each canonical element, OP2's first levels, back into the tile.
 template <int OP1, int OP2, int R, class Step>
@@ -622,133 +591,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_butterfly_strided(const Fe*
 // Two transforms on the same tile bits, with a step on the canonical values
 // in between, in one trip through HBM.  The transforms are tensor products of
 // 2 x 2 maps on the index bits, so the levels of either one can run in any
-// order and levels on different bits commute: a pass may take the message's
-// Mobius levels on bits [lo, lo + k) and then the first WHT's levels on the
-// same bits, or the first WHT's last levels, the alpha product and the second
-// WHT's first levels.
-
-// Registers -> planes: v[j] is tile element base + (j << zb).
-template <int R>
-__device__ __forceinline__ void regs_to_planes(uint32_t* planes, int base, int zb, const uint32_t (&v)[1 << R][kC]) {
-  const int pb = pidx(base);
-#pragma unroll
-  for (int j = 0; j < (1 << R); ++j) {
-    const int q = pb ^ pidx(j << zb);
-#pragma unroll
-    for (int c = 0; c < kC; ++c) planes[c * kPlane + q] = v[j][c];
-  }
-}
-
-// Planar levels on tile bits [b0, 6) of a full tile (the levels between a
-// register head on bits 9..11 and a register tail on bits 6..8), lvl0 the
-// first level's lazy index.  A radix-4 stage on bits 4..5 takes its groups
-// with bits 4 and 5 swapped (conflict-free banks, see tile_loop).
-template <int OP>
-__device__ __forceinline__ void fused_middle(uint32_t* planes, int b0, int lvl0) {
-  if (b0 == 4) planar_stage<OP, 2, true>(planes, kMaxTileLog, 4, lvl0);
-  else planar_levels<OP>(planes, kMaxTileLog, b0, 6 - b0, lvl0);
-}
-
-// Runs OP1 on tile bits [b0, 12) of full 4096-element tiles, then for each
-// element mid(tile, t, Fr& v) on its canonical value, then OP2 on the same
-// bits, then st(tile, t, uint4).  512 threads, 6 >= b0 >= 0.  OP1: register
-// head on bits 9..11, planar levels on [b0, 6), register tail on bits 6..8;
-// mid on the tail's registers; OP2: register levels on bits 6..8 right
-// there, planar levels on [b0, 6), register tail on bits 9..11 and the
-// stores (consecutive threads take consecutive elements, as the loads).
-// stage(tile) runs first in each tile (to issue its cp.async side loads,
-// which each thread then waits for before the first planar stage's barrier).
-// The tile's 16-byte elements (src(tile, t)) arrive by cp.async in a staging
-// area of kPrefetchSmem bytes after the planes: thread g copies elements
-// g + (j << 9) and reads back only its own copies, so the next tile's copies
-// are issued right after the head and land while the rest of the tile runs,
-// without holding registers.  Commit groups per tile: the side loads and an
-// always-present group closing them, then the next tile's elements.
-constexpr size_t kPrefetchSmem = size_t(1) << kMaxTileLog << 4;  // 64 KiB
-template <int OP1, int OP2, class Src, class Conv, class Stage, class Mid, class St>
-__device__ __forceinline__ void tile_loop_fused(uint32_t* planes, int b0, uint32_t n_tiles, Src src, Conv conv,
-                                                Stage stage, Mid mid, St st) {
-  const int g = threadIdx.x;
-  const int rm = 6 - b0;
-  const int tb = (g & 63) | ((g >> 6) << 9);  // the tail group: elements tb + (j << 6)
-  uint4* pre = reinterpret_cast<uint4*>(planes + kC * kPlane);
-  uint32_t tile = blockIdx.x;
-  if (tile < n_tiles)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) cp_async16(pre + g + (j << 9), src(tile, g + (j << 9)));
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (; tile < n_tiles; tile += gridDim.x) {
-    stage(tile);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // this tile's elements (and older groups) have landed
-    {
-      uint32_t v[8][kC];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const Fr e = conv(tile, g + (j << 9), pre[g + (j << 9)]);
-#pragma unroll
-        for (int c = 0; c < kC; ++c) v[j][c] = e.c[c];
-      }
-      head_levels<OP1>(planes, v);
-    }
-    const uint32_t next = tile + gridDim.x;
-    if (next < n_tiles)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) cp_async16(pre + g + (j << 9), src(next, g + (j << 9)));
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // the side loads; the next tile's copies may pend
-    if (rm > 0) fused_middle<OP1>(planes, b0, 3);
-    else __syncthreads();
-    {
-      uint32_t v[8][kC];
-      const int pb = pidx(tb);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int q = pb ^ pidx(j << 6);
-#pragma unroll
-        for (int c = 0; c < kC; ++c) v[j][c] = planes[c * kPlane + q];
-      }
-      reg_levels<OP1, 3>(v, 3 + rm);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        Fr w;
-#pragma unroll
-        for (int c = 0; c < kC; ++c) w.c[c] = tile_final(v[j][c]);
-        mid(tile, tb + (j << 6), w);
-#pragma unroll
-        for (int c = 0; c < kC; ++c) v[j][c] = w.c[c];
-      }
-      reg_levels<OP2, 3>(v, 0);
-      // The same thread read these positions: no other thread touches them
-      // until the barrier below.
-      regs_to_planes<3>(planes, tb, 6, v);
-    }
-    __syncthreads();
-    if (rm > 0) fused_middle<OP2>(planes, b0, 3);
-    auto st_t = [&](int t, uint4 u) { st(tile, t, u); };
-    pass_tail<OP2, 3>(planes, 9, 3 + rm, st_t);
-    __syncthreads();  // the next head overwrites the planes
-  }
-}
-
-// Message half at cw: Mobius levels [lo, lo + k) (the message is final after
-// them), stored back; then the first WHT's levels [lo, lo + k) of the same
-// values, stored into the parity half at cw + R.  k in [6, 10], cb = 12 - k
-// (or 2 at k = 10).
-__global__ void __launch_bounds__(kTileThreads, 1) k_mobius_wht_strided(Fe* cw, uint32_t R, int logR, int lo, int k, int cb,
-                                                                       uint32_t n_tiles) {
-  extern __shared__ uint32_t planes_s[];
-  auto src = [=](uint32_t tile, int t) -> const void* { return cw + strided_addr(tile, t, logR, lo, k, cb); };
-  auto conv = [](uint32_t, int, uint4 raw) { return unpack_fe(raw); };
-  auto stage = [](uint32_t) {};
-  auto mid = [=](uint32_t tile, int t, Fr& v) {
-    *reinterpret_cast<uint4*>(cw + strided_addr(tile, t, logR, lo, k, cb)) = pack_fe(v);
-  };
-  auto st = [=](uint32_t tile, int t, uint4 u) {
-    *reinterpret_cast<uint4*>(cw + R + strided_addr(tile, t, logR, lo, k, cb)) = u;
-  };
-  tile_loop_fused<kMobius, kWht>(planes_s, cb, n_tiles, src, conv, stage, mid, st);
-}
+// order and levels on different bits commute: a pass takes the first WHT's last
+// levels, the alpha product and the second WHT's first levels.
 
 // The parity tile pass: the first WHT's levels 0..11 of each column (read at
 // src, the message half when no strided WHT level came first, else the

@@ -92,8 +92,8 @@ struct TcLayout {
     }
     return u | (e >> n(3) & 1u) << 8;
   }
-  // Slots of epilogue lane m (the contracted output index), of column group
-  // n (16 per chunk) and of chunk c.
+  // Slots of epilogue lane m (the contracted output index) and of column group
+  // n (16 per chunk).
   static constexpr uint32_t of_m(uint32_t m) {
     uint32_t e = 0;
     for (int i = 0; i < 7; ++i) e |= (m >> i & 1u) << k(i);
@@ -104,7 +104,6 @@ struct TcLayout {
     for (int i = 0; i < 4; ++i) e |= (v >> i & 1u) << n(i);
     return e;
   }
-  static constexpr uint32_t of_chunk(uint32_t c) { return (c & 1u) << chunk(0) | (c >> 1) << chunk(1); }
 };
 
 // Codeword index of tile `tile`'s element 0: the tile numbers the index bits
