@@ -743,10 +743,10 @@ def main():
         pairs = {"eo_witness": ("k_eo_witness_mma", "k_eo_witness"), "block_fold": ("k_block_fold_mma", "k_block_fold"),
                  "eq_projection": ("k_eq_project_mma", "k_eq_project_tc")}
         imma_cmp = {}
-        for name, (on_k, off_k) in pairs.items():
+        for weight_pass, (on_k, off_k) in pairs.items():
             a, b = on_stats.get(on_k), off.get(off_k)
             if a and b:
-                imma_cmp[name] = {"imma_ms": a["ms"], "dp4a_ms": b["ms"], "speedup": b["ms"] / a["ms"],
+                imma_cmp[weight_pass] = {"imma_ms": a["ms"], "dp4a_ms": b["ms"], "speedup": b["ms"] / a["ms"],
                                   "imma_hbm_frac": a["bytes"] / (a["ms"] / 1000.0) / 1e9 / peak,
                                   "dp4a_hbm_frac": b["bytes"] / (b["ms"] / 1000.0) / 1e9 / peak}
         imma_cmp["what"] = ("per-step kernel time of the exact integer-limb tensor-core kernels (mma.sync s8 x u8 -> "
