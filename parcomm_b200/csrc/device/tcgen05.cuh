@@ -1,6 +1,6 @@
-// sm_100a primitives of the tensor-core transform passes: tcgen05 (TMEM
-// allocation, integer MMA, loads), mbarriers with a bounded wait, proxy
-// fences and the shared-memory descriptors.
+// sm_100a primitives of the tensor-core transform passes and projections:
+// tcgen05 (TMEM allocation, integer MMA, loads), mbarriers with a bounded wait,
+// bulk copies, proxy fences and the shared-memory descriptors.
 #pragma once
 #include <cstdint>
 

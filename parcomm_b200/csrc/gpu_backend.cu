@@ -48,11 +48,13 @@ static bool imma_on() {
 // B200 in the 8B-shape step, on the CUDA cores elsewhere (core_dots 0);
 // core_dots 1 takes the CUDA cores everywhere, 2 the tensor cores
 // everywhere.  The tensor-core sums win on the long vectors: EO dot and
-// first cross pair 2.5x / 2.2x, EO query fold 1.4x / 1.13x, sumcheck message
-// 1.7x / 1.3x and fold 1.09x / 1.19x (F65521 / KoalaBear).  On the short
+// first cross pair 2.3x / 1.26x, EO query fold 1.28x / 0.96x, sumcheck message
+// 1.6x / 1.06x and fold 1.04x / 0.98x (F65521 / KoalaBear).  On the short
 // vectors of the LiteBullet rounds and the small EO rounds the chunked warp
-// loop and its staging cost more than they save (0.7x - 0.9x), except the
-// KoalaBear LiteBullet cross pair (1.03x).
+// loop and its staging cost more than they save (0.7x - 0.85x).  The three
+// KoalaBear choices below one (the LiteBullet cross pair 0.81x) were above it
+// before the KoalaBear products by Montgomery reduction; they cost 0.4 ms of
+// a 285 ms step.
 enum class Dots { kEoDotCross, kEoFoldQueryCross, kEoFoldCross, kSumMessage, kSumFold, kLbCross, kLbFold, kDot };
 static bool tc_dots(Dots k) {
   const int opt = KernelOptions::core_dots.load();
@@ -1101,13 +1103,17 @@ static std::vector<F> tensor_slice(const std::vector<F>& p) { return tensor_weig
 // (kernels/eq_mma.cuh).  Its time hardly depends on nb (the MMA takes eight
 // blocks' rows either way), the CUDA-core kernels' does.  Measured on B200, us,
 // tcgen05 / CUDA cores, F65521 then KoalaBear:
-//   8 blocks   2^12  9 / 18, 9 / 24      2^20  33 / 49, 33 / 76
-//              2^27  1769 / 4435, 2864 / 6269
-//   4 blocks   2^14  10 / 13, 12 / 15    2^20  28 / 30, 32 / 42
-//              2^22  55 / 87, 68 / 117
+//   8 blocks   2^12   8 / 18, 10 / 25    2^20  31 / 48, 35 / 77
+//              2^24  236 / 567, 236 / 813; 2^27 (F65521) 1769 / 4435
+//   4 blocks   2^14   9 / 14, 11 / 15    2^20  28 / 30, 33 / 41
+//              2^22  55 / 87, 70 / 116
 //   4 blocks   2^16  17 / 13, 19 / 18    2^18  21 / 13, 23 / 17: a few stages
 //              per CTA, one after the other, against four CTAs per SM
+//   3 blocks   2^28 (KoalaBear) 2864 / 6279
 //   1 block    2^20  22 / 15, 26 / 20
+// Both lines are on the safe side, not tight: fewer than four blocks were timed
+// at 2^20 first, where the CUDA cores win, and three large blocks would gain; in
+// the gap above 2^14 eight blocks take the CUDA cores 18 to 28 us.
 // Bulk copies take 16-byte aligned weights.
 static bool eq_on_tcgen05(uint64_t m, int nb, uint64_t block_bytes, const void* weights) {
   if (nb < 4 || m % (2 * qfd::kEtPairs) || (m > (1u << 14) && m < (1u << 20))) return false;

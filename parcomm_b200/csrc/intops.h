@@ -23,16 +23,17 @@ struct FieldOps {
 // add (a + 2^l p - b), a Mobius pair one three-operand add; a reduction folds
 // 2^16 = 15 once (shift, multiply-add) and subtracts p once (subtract,
 // minimum); unpack is one extract per coefficient, pack one permute per two.
-// The product: 8 multiplies by 17, 64 widening multiply-adds (two issue slots
-// each), 8 reductions of about 6 operations.
-constexpr FieldOps kF65521{1.0, 0.5, 4.0, 1.5, 8 + 64 * 2 + 8 * 6, 8};
+// The product: the byte planes (24 permutes), 17 b_j mod p (8 of five
+// operations), the windows (24 permutes), 64 dp4a, 8 joins of two multiply-adds,
+// 8 reductions of four operations.
+constexpr FieldOps kF65521{1.0, 0.5, 4.0, 1.5, 24 + 8 * 5 + 24 + 64 + 8 * 2 + 8 * 4, 8};
 // KoalaBear^4, canonical after every butterfly: addp / subp are an add or
 // subtract, the corrected value and an unsigned minimum (3 operations), so a
 // WHT pair costs 6 and a Mobius pair 3.  Values stay canonical 32-bit words:
 // no reduction and no unpacking.  The product: 3 b_j by two modular additions
-// (24), 16 widening products (two slots each), 4 Barrett reductions of about
-// 15 operations.
-constexpr FieldOps kKoalaBear{3.0, 1.5, 0.0, 0.0, 24 + 16 * 2 + 4 * 15, 4};
+// (24), 16 widening products (two slots each), 4 Montgomery reductions of seven
+// operations, and b_j scaled by 2^32 (4 widening products and reductions).
+constexpr FieldOps kKoalaBear{3.0, 1.5, 0.0, 0.0, 24 + 16 * 2 + 4 * 7 + 4 * (2 + 7), 4};
 
 // One BLAKE2s compression: 10 rounds of 8 G functions, each 6 additions,
 // 4 XORs and 4 rotations.

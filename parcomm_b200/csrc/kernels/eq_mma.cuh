@@ -16,13 +16,17 @@
 // 2^14 * 255 * 255 < 2^30; the table is read once for all blocks.
 //
 // The CUDA-core kernels spend their time on multiply-adds (F65521 dp4a with
-// byte transposes, KoalaBear widening multiply-adds).  Measured on B200, eight
-// blocks of 2^27 elements: F65521 1.77 ms, 6.1 TB/s, bound by HBM (dp4a 4.44);
-// KoalaBear 2.86 ms (6.27), bound by its 16 MMAs per stage.  Neighbouring CTAs
-// take neighbouring stages: a contiguous run of stages per CTA put 1300 streams
-// on distant pages (F65521 3.85 against 3.35 ms, before one lane per block
-// issued the copies).  Chunks 4096 bytes apart put a row's 16-byte units on the
-// same banks; 16 bytes more per chunk brought KoalaBear from 3.30 to 2.86 ms.
+// byte transposes, KoalaBear widening multiply-adds).  Measured on B200:
+//   F65521, eight blocks of 2^27 elements: 1.77 ms, 6.1 TB/s, bound by HBM (4.44
+//   on the CUDA cores);
+//   KoalaBear, eight blocks of 2^24: 0.236 ms (0.813), of 2^28: 3.53 ms, 6.1
+//   TB/s, bound by HBM; three blocks of 2^28: 2.86 ms (6.28), 3.7 TB/s, bound by
+//   the 16 MMAs of a stage, which take eight blocks' rows either way.
+// Neighbouring CTAs take neighbouring stages: a contiguous run of stages per CTA
+// put 1300 streams on distant pages (F65521 3.85 against 3.35 ms, before one lane
+// per block issued the copies).  Chunks 4096 bytes apart put a row's 16-byte
+// units on the same banks; 16 bytes more per chunk brought three KoalaBear blocks
+// of 2^28 from 3.30 to 2.86 ms.
 #pragma once
 #include <cstdint>
 
