@@ -388,13 +388,20 @@ static void wht_tile_launch(cudaStream_t s, const Fe* src, Fe* dst, const Fe* al
 
 // Codewords of fewer than 2^19 message entries have fewer 4096-element tiles
 // than the chip has SMs, and a pass takes as long as one tile: their tiles
-// shrink to 1/128 of the message.  Up to 2^12 entries one tile takes the whole
-// Mobius transform in one launch, and a second launch costs more than the
-// smaller tiles save (root of one F65521 block, us, one tile / 64-element tiles
-// and a second pass: 2^7 36.4 / 40.5, 2^10 45.1 / 47.4, 2^12 52.0 / 52.2; at 2^13
-// two passes are needed either way, 67.7 / 59.4).
+// shrink to 1/128 of the message.  Few entries stay in one tile, which takes the
+// whole Mobius transform in one launch: a second launch costs more than the
+// smaller tiles save.  Commitment of 32 blocks, us per block, one tile /
+// 64-element tiles and a second pass: F65521 2^7 63.7 / 66.3, 2^10 74.1 / 76.5,
+// 2^11 75.6 / 76.7, 2^12 79.8 / 78.7; KoalaBear (half as many coefficients) 2^8
+// 63.1 / 66.3, 2^12 75.4 / 76.9.  At 2^13 two passes are needed either way (root
+// of an F65521 block 67.7 / 59.4).
+#if defined(QF_FIELD_KB)
+static constexpr int kOneTileLog = 12;
+#else
+static constexpr int kOneTileLog = 11;
+#endif
 static int small_tile_log(int logm) {
-  return logm <= qfd::kMaxTileLog ? logm : std::min(qfd::kMaxTileLog, std::max(6, logm - 7));
+  return logm <= kOneTileLog ? logm : std::min(qfd::kMaxTileLog, std::max(6, logm - 7));
 }
 
 // 2^cb consecutive group bases per tile of a k-level strided pass: 64-byte

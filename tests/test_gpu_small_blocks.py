@@ -1,5 +1,5 @@
-"""Blocks of 2^7 to 2^14 packed elements, around the size up to which one tile
-takes the whole Mobius transform (2^12): roots, claims and proofs against the
+"""Blocks of 2^7 to 2^14 packed elements, around the sizes up to which one tile
+takes the whole Mobius transform (2^11, KoalaBear 2^12): roots, claims and proofs against the
 oracle, and the root of each block without allocation.  Needs a B200."""
 import numpy as np
 import pytest
